@@ -513,9 +513,11 @@ struct CflStepFinish {
         H.outer[k] = pcg_mixed ? P->outer : 0;
         // the step's 10 kernels and the PCG's: init + 3 per iteration in the FP64 forms
         // (2 with AMG, whose V-cycle and direction kernels count themselves on the device),
-        // all counted on the device in the mixed form
+        // all counted on the device in the mixed form; 1 where the solve is one launch
         H.kernels[k] = 10 + H.stamp_kernels +
-                       (pcg_mixed ? P->kernels : 1 + (P->kernels ? 2 : 3) * P->iter + P->kernels);
+                       (pcg_mixed         ? P->kernels
+                        : P->one_launch ? 1
+                                        : 1 + (P->kernels ? 2 : 3) * P->iter + P->kernels);
       }
       S->step = k + 1;
     }

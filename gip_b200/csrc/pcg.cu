@@ -62,6 +62,7 @@ struct PcgInitFinish {
     S->rr = t[1];
     S->bb = t[2];
     S->iter = 0;
+    S->one_launch = 0;
     S->status = GIPB200_OK;
     S->done = (maxit <= 0) ? 1 : 0;
     if (mode == GIPB200_PCG_TOL && !(sqrt(t[1]) > tol * sqrt(t[2]))) S->done = 1;
@@ -922,7 +923,9 @@ int Pcg::init(const Sell* Lm, int nall, const gipb200_pcg_params& params, cudaSt
   } else {
     GIPB_TRY(dinv.alloc(n));
     GIPB_TRY(p.alloc(n_all));
+    GIPB_TRY(p.zero(s));
     GIPB_TRY(Ap.alloc(n));
+    GIPB_TRY(Ap.zero(s));
     GIPB_TRY(r.alloc(n));
     if (n > 0) {
       DevBuf<int> miss;
@@ -935,6 +938,7 @@ int Pcg::init(const Sell* Lm, int nall, const gipb200_pcg_params& params, cudaSt
       GIPB_CUDA(cudaStreamSynchronize(s));
     }
     if (prm.precond == GIPB200_PRECOND_AMG) GIPB_TRY(build_amg64(s));
+    GIPB_TRY(plan_one_launch(s));
   }
   GIPB_CUDA(cudaStreamSynchronize(s));
   return GIPB200_OK;
@@ -1270,7 +1274,7 @@ double Pcg::iteration_bytes() const {
     if (amg) b += amg->cycle_bytes(cop.enabled ? cop.bytes_per_launch - 16.0 * nn : plain);
     return b;
   }
-  const double spmv = 12.0 * nnz + 16.0 * nn;
+  const double spmv = (op64.bits ? packed64_bytes() : 12.0 * nnz) + 16.0 * nn;
   if (amg64) {  // update (x, r read and written; p, Ap read), cycle, p = z + beta p
     const double a0 = (double)L->nslots * 12.0 + (L->nslices + 1.0) * 8.0;
     return spmv + 48.0 * nn + amg64->cycle_bytes(a0) + 24.0 * nn;
@@ -1363,6 +1367,7 @@ static int host_poll_interval() {
 }
 
 int Pcg::enqueue(const double* b, double* x, const double* x0, cudaStream_t s, bool host_sync) {
+  if (one_launch()) return enqueue_one_launch(b, x, x0, s);
   if (!host_sync && prm.mode != GIPB200_PCG_FIXED && capturing(s)) {
     if (!body_stream[0]) {
       return fail(GIPB200_ERR_STATE, "capture streams missing");
@@ -1386,6 +1391,13 @@ void Pcg::launch_pcg_update(double* x, cudaStream_t s) {
                                                    prm.mode, prm.maxit, prm.tol);
 }
 
+void Pcg::launch_pcg_spmv(cudaStream_t s) {
+  if (op64.bits)
+    launch_packed64_spmv(Ap.p, sc.p, prm.mode, s);
+  else
+    k_pcg_spmv_dot<<<blocks_spmv, 256, 0, s>>>(L->view(), p.p, Ap.p, sc.p, rs, prm.mode);
+}
+
 int Pcg::enqueue_fp64_graph(const double* b, double* x, const double* x0, cudaStream_t s) {
   cudaGraphConditionalHandle h;
   GIPB_TRY(make_handle(s, 0, 0, &h));
@@ -1404,7 +1416,7 @@ int Pcg::enqueue_fp64_graph(const double* b, double* x, const double* x0, cudaSt
   cudaStream_t bs = body_stream[0];
   GIPB_CUDA(cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0,
                                           cudaStreamCaptureModeRelaxed));
-  k_pcg_spmv_dot<<<blocks_spmv, 256, 0, bs>>>(L->view(), p.p, Ap.p, sc.p, rs, prm.mode);
+  launch_pcg_spmv(bs);
   int ast = GIPB200_OK;
   if (amg64) {
     k_pcg_update_amg<<<blocks_vec, 256, 0, bs>>>(n, x, r.p, p.p, Ap.p, sc.p, rs, prm.maxit, prm.tol);
@@ -1517,7 +1529,7 @@ int Pcg::enqueue_fp64(const double* b, double* x, const double* x0, cudaStream_t
   }
   const int poll = host_poll_interval();
   for (int k = 0; k < prm.maxit; ++k) {
-    k_pcg_spmv_dot<<<blocks_spmv, 256, 0, s>>>(L->view(), p.p, Ap.p, sc.p, rs, prm.mode);
+    launch_pcg_spmv(s);
     if (amg64) {
       k_pcg_update_amg<<<blocks_vec, 256, 0, s>>>(n, x, r.p, p.p, Ap.p, sc.p, rs, prm.maxit,
                                                    prm.tol);
@@ -1695,6 +1707,8 @@ int Pcg::time_spmv(int mixed, int reps, cudaStream_t s, double* avg_ms, double* 
     if (k == 1) GIPB_CUDA(cudaEventRecord(e0, s));
     if (mixed)
       launch_mx_spmv(*this, p32.p, p32b.p, Ap32.p, tAp32.p, tsc.p, 0, 0, s);
+    else if (op64.bits)
+      launch_packed64_spmv(tAp.p, tsc.p, GIPB200_PCG_FIXED, s);
     else
       k_pcg_spmv_dot<<<blocks_spmv, 256, 0, s>>>(L->view(), p.p, tAp.p, tsc.p, rs,
                                                   GIPB200_PCG_FIXED);
@@ -1713,6 +1727,7 @@ int Pcg::time_spmv(int mixed, int reps, cudaStream_t s, double* avg_ms, double* 
   *bytes = (double)L->nnz * (vbytes + 4.0) + (double)(L->nslices + 1) * 8.0 +
            (double)L->nrows * (mixed ? 4.0 : 2.0) * vbytes;
   if (mixed && cop.enabled) *bytes = cop.bytes_per_launch;
+  if (!mixed && op64.bits) *bytes = packed64_bytes() + 16.0 * L->nrows;
   if (mixed && rec) *bytes += 4.0 * L->nrows;  // the previous A p, read by the recurrence
   return GIPB200_OK;
 }

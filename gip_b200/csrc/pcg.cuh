@@ -24,7 +24,7 @@ struct PcgScalars {
   int outer;        // MIXED: refinement cycles done
   int total_inner;  // MIXED: inner iterations summed over cycles
   int kernels;      // MIXED: PCG kernel launches of this solve, early exits included
-  int pad1;
+  int one_launch;   // FP64 modes: the solve ran as one kernel
   double rsum;      // MIXED: sum of the FP64 residual (pinned-Neumann deflation)
   double kappa_c;   // MIXED: sum(r)/pin of the current segment
   double kappa;     // MIXED: constant added to x at the next replacement
@@ -54,6 +54,28 @@ struct CompressedOp {
   int ntable = 0;
   double compressed_fraction = 0.0;  // share of L's slots in packed slices
   double bytes_per_launch = 0.0;     // stored bytes the kernel streams (+ vectors)
+};
+
+// The FP64 operator packed in GIP's slot order (build_packed64); bits = 0: not built.
+struct Packed64 {
+  int bits = 0;                  // value-table index bits: 4 or 8
+  DevBuf<uint4> delta;
+  DevBuf<unsigned> idx4;
+  DevBuf<uint2> idx8;
+  DevBuf<int> base;
+  DevBuf<unsigned char> plain;
+  DevBuf<double> table;
+};
+
+// How a whole FP64 Jacobi solve runs as one launch (persist.cu); kNone: kernel by kernel.
+struct OneLaunch {
+  enum { kNone = 0, kCluster, kGrid, kStream };
+  int form = kNone;
+  int ctas = 0, threads = 0;
+  int per_thread = 1;            // register forms: rows per thread
+  size_t shared = 0;             // dynamic shared memory per CTA
+  DevBuf<double2> pair;          // kGrid: (z, p) of every row
+  DevBuf<ulonglong2> slots;      // grid reductions
 };
 
 struct Pcg {
@@ -121,6 +143,14 @@ struct Pcg {
   // constant mode is restored exactly from the pin equation.
   int pin_row = -1;
   double pin_val = 0.0;
+  Packed64 op64;
+  OneLaunch one;
+  // several solvers advance side by side on one GPU (a batch): forms that claim every SM at
+  // once (the cooperative ones) would take turns, so only the cluster form runs
+  bool shared_gpu = false;
+  bool one_launch() const {
+    return one.form == OneLaunch::kCluster || (one.form != OneLaunch::kNone && !shared_gpu);
+  }
   // scalars and reduction scratch
   DevBuf<PcgScalars> sc;
   DevBuf<double> partials;
@@ -152,6 +182,14 @@ struct Pcg {
   int vcycle_forms(int cap, int* n_kernels, int* h_form) const;
 
  private:
+  int build_packed64(cudaStream_t s);
+  int plan_one_launch(cudaStream_t s);
+  void launch_packed64_spmv(double* q, PcgScalars* S, int mode, cudaStream_t s);
+  // operator bytes a product streams from the packed FP64 layout: column deltas, value
+  // indices, the slices' slot bases
+  double packed64_bytes() const { return (16.0 + op64.bits) * n + 33.0 * L->nslices; }
+  void launch_pcg_spmv(cudaStream_t s);  // A p and p.Ap of the three-kernel loop
+  int enqueue_one_launch(const double* b, double* x, const double* x0, cudaStream_t s);
   int enqueue_fp64(const double* b, double* x, const double* x0, cudaStream_t s, bool host_sync);
   int enqueue_mixed(const double* b, double* x, const double* x0, cudaStream_t s, bool host_sync);
   int read_flag(cudaStream_t s, int which, int* v);

@@ -1,0 +1,769 @@
+// FP64 Jacobi-PCG (GIP_LinearSolver::solve, src/Algorithms/GIP_LinearSolver.h:44-117) as one
+// launch.
+//
+// The three-kernel loop of pcg.cu spends a launch, a drain and a ticket reduction per kernel:
+// 4.1 us each on the 12^3 cavity, whose work is a fraction of a microsecond.  Here the whole
+// solve is one kernel whose CTAs stay resident, and an iteration is
+//   A: Ap = L p with p_j = z_j + beta p_j formed where it is gathered (the IEEE operations
+//      of the separate update, so the same values)                       -> p.Ap, alpha
+//   B: x += alpha p, r -= alpha Ap, z = dinv r, (z, p) published           -> r.z, r.r, beta
+// with two reductions over all CTAs and no other barrier.  Every row belongs to one thread
+// for the whole solve, which keeps x, r, p, dinv and the row's operator in registers; only
+// the pair (z, p) of a row is ever written, for the threads that gather it.
+//   cluster form: up to 16384 rows (16 CTAs of 256 threads, 4 rows each), the pairs in the
+//     cluster's shared memory, the reductions over hardware cluster barriers;
+//   grid form: up to 4 rows per thread of 256 on every SM (151552 rows on 148 SMs), the pairs
+//     in global memory (L2), the reductions over epoch-stamped slots (persist.cuh);
+//   streamed form: more rows, while r and Ap fit the SMs' shared memory (2.1 million rows on
+//     148 SMs), for operators that pack; below.
+// Measured per iteration against the three-kernel loop inside a step graph (host-driven it
+// took 20 us or more): 12^3 2.6 against 12.2 us (cluster of 4; the grid form 4.9), 24^3 4.2
+// (cluster of 16; grid 5.2), 48^3 6.0 against 16.7 (streamed 9.1), 64^3 10.6 against 23
+// (host-driven), 128^3 32.5 against 84.
+// Element operations are GIP's (no FMA contraction); only the order of the dot products' sums
+// differs from the other forms.  Columns of ghost cells hold stored zeros in these operators
+// (checked at set-up): they enter the initial residual like every column, and the iterations,
+// where their entries of p stay fixed, drop them.
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <vector>
+
+#include "persist.cuh"
+
+namespace gipb200 {
+namespace {
+
+constexpr int kRowSlots = 8;  // longest row of the register forms
+
+struct Args64 {
+  SellView<double> L;
+  const double* b;
+  const double* x0;
+  const double* dinv;
+  double* x;
+  double2* pair;      // grid form: (z, p) of every row
+  ulonglong2* slots;  // grid forms: reduction slots (zero at launch)
+  PcgScalars* S;
+  double tol;
+  int n, n_all, mode, maxit;
+};
+
+// The solve's scalars, held identically by every thread.
+struct Scal64 {
+  double rz, pAp, alpha, beta, rr, bb;
+  int iter, done, status;
+};
+
+// After the initial residual (PcgInitFinish of the three-kernel loop).
+__device__ __forceinline__ void start64(Scal64& T, const double (&t)[3], int mode, int maxit,
+                                        double tol) {
+  T.rz = t[0];
+  T.rr = t[1];
+  T.bb = t[2];
+  T.pAp = T.alpha = T.beta = 0.0;
+  T.iter = 0;
+  T.status = GIPB200_OK;
+  T.done = (maxit <= 0) ? 1 : 0;
+  if (mode == GIPB200_PCG_TOL && !(sqrt(t[1]) > tol * sqrt(t[2]))) T.done = 1;
+  if (mode != GIPB200_PCG_FIXED && !(isfinite(t[1]) && isfinite(t[2]))) {
+    T.status = GIPB200_ERR_BREAKDOWN;
+    T.done = 1;
+  }
+}
+
+// After p.Ap; false: breakdown, the iteration ends before its update.
+__device__ __forceinline__ bool alpha64(Scal64& T, double pAp, int mode) {
+  T.pAp = pAp;
+  T.alpha = ddiv(T.rz, pAp);
+  if (mode != GIPB200_PCG_FIXED && (!(pAp > 0.0) || !isfinite(T.alpha))) {
+    T.status = GIPB200_ERR_BREAKDOWN;
+    T.done = 1;
+    return false;
+  }
+  return true;
+}
+
+// After r.z and r.r.
+__device__ __forceinline__ void beta64(Scal64& T, const double (&t)[2], int mode, int maxit,
+                                       double tol) {
+  const double r0 = T.rz;
+  T.rz = t[0];
+  T.rr = t[1];
+  T.beta = ddiv(t[0], r0);
+  T.iter += 1;
+  if (mode == GIPB200_PCG_TOL && !(sqrt(t[1]) > tol * sqrt(T.bb))) T.done = 1;
+  if (T.iter >= maxit) {
+    if (mode == GIPB200_PCG_TOL && !T.done) T.status = GIPB200_ERR_NOT_CONVERGED;
+    T.done = 1;
+  }
+}
+
+__device__ __forceinline__ void store64(PcgScalars* S, const Scal64& T) {
+  S->rz = T.rz;
+  S->pAp = T.pAp;
+  S->alpha = T.alpha;
+  S->beta = T.beta;
+  S->rr = T.rr;
+  S->bb = T.bb;
+  S->iter = T.iter;
+  S->done = 1;
+  S->status = T.status;
+  S->kernels = 0;
+  S->one_launch = 1;
+}
+
+// ------------------------------------------------------------------ register forms
+// Where a row's (z, p) pair lives and how the sums travel.
+struct ClusterPairs {
+  static constexpr int kMaxCtas = 16;
+  unsigned rank, size;
+  int rows;                  // rows of one CTA
+  unsigned pairs;            // shared address of this CTA's pairs
+  double (*red)[3][8 * kMaxCtas];  // [parity][sum][warp of the cluster]
+  int par = 0;
+  __device__ __forceinline__ unsigned where(int row) const {
+    return map_shared(pairs + 16u * (unsigned)(row % rows), (unsigned)(row / rows));
+  }
+  __device__ __forceinline__ double2 load(unsigned a) const {
+    double2 v;
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    return v;
+  }
+  __device__ __forceinline__ void publish(int row, double z, double p) const {
+    asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(pairs + 16u * (unsigned)(row - (int)rank * rows)),
+                 "d"(z), "d"(p)
+                 : "memory");
+  }
+  // Each warp sends its partial sums to every CTA; after one barrier every warp adds all of
+  // them in the same order.  The barrier also publishes the pairs.
+  template <int W, bool FENCE>
+  __device__ __forceinline__ bool sum(double (&v)[W]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const double t = warp_reduce<SumOp>(v[k]);
+      if (lane < (int)size)
+        st_cluster(map_shared(smem_u32(&red[par][k][rank * nw + warp]), (unsigned)lane), t);
+    }
+    if (size == 1u) __syncthreads();  // (a cluster barrier costs 370 cycles, this 30)
+    else cluster_barrier();
+    const int total = nw * (int)size;
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      double a = 0.0;
+      for (int i = lane; i < total; i += 32) a = dadd(a, red[par][k][i]);
+      v[k] = warp_reduce<SumOp>(a);
+    }
+    par ^= 1;
+    return true;
+  }
+};
+
+struct GridPairs {
+  double2* pairs;
+  GridScope G;
+  __device__ __forceinline__ int where(int row) const { return row; }
+  // plain loads: the reduction that published the pairs is an acquire for the whole CTA
+  __device__ __forceinline__ double2 load(int row) const { return pairs[row]; }
+  __device__ __forceinline__ void publish(int row, double z, double p) const {
+    pairs[row] = make_double2(z, p);
+  }
+  template <int W, bool FENCE>
+  __device__ __forceinline__ bool sum(double (&v)[W]) {
+    return grid_sum<W, FENCE>(v, G);
+  }
+};
+
+// K rows per thread: rows first + k * blockDim.x + threadIdx.x of the CTA's K * blockDim.x.
+template <int K, class Pairs>
+__device__ __forceinline__ void solve_rows(const Args64& A, Pairs& Q, int rank, int ncta) {
+  using Addr = decltype(Q.where(0));
+  const int lane = threadIdx.x & 31;
+  const int i0 = rank * K * (int)blockDim.x + (int)threadIdx.x;
+  // the rows' operator and the initial residual r = b - L x0, z = dinv r, p = z
+  Addr at[K][kRowSlots];
+  double v[K][kRowSlots];
+  double x[K], r[K], z[K], p[K], q[K], di[K];
+  double acc3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = i0 + k * (int)blockDim.x;
+    const bool own = i < A.n;
+    long long base = 0;
+    int len = 0;
+    const int s = i >> 5;
+    if (s < A.L.nslices) slice_range(A.L, s, base, len);
+    double sum = 0.0;
+#pragma unroll
+    for (int j = 0; j < kRowSlots; ++j) {
+      const int c = (j < len) ? A.L.col[base + 32LL * j + lane] : -1;
+      v[k][j] = (c >= 0) ? A.L.val[base + 32LL * j + lane] : 0.0;
+      if (c >= 0) sum = dadd(sum, dmul(A.x0[c], v[k][j]));
+      // padding and ghost columns: the row's own pair times a zero
+      at[k][j] = Q.where((c >= 0 && c < A.n) ? c : (own ? i : 0));
+    }
+    x[k] = r[k] = z[k] = p[k] = q[k] = di[k] = 0.0;
+    if (own) {
+      const double bi = A.b[i];
+      x[k] = A.x0[i];
+      di[k] = A.dinv[i];
+      r[k] = dadd(bi, dmul(-1.0, sum));
+      z[k] = dadd(0.0, dmul(r[k], di[k]));
+      acc3[0] = dadd(acc3[0], dmul(r[k], z[k]));
+      acc3[1] = dadd(acc3[1], dmul(r[k], r[k]));
+      acc3[2] = dadd(acc3[2], dmul(bi, bi));
+      Q.publish(i, z[k], 0.0);
+    }
+  }
+  Scal64 T;
+  bool ok = Q.template sum<3, true>(acc3);
+  start64(T, acc3, A.mode, A.maxit, A.tol);
+  if (A.x != A.x0)  // (after the reduction: every row has read x0)
+    for (int g = A.n + rank * (int)blockDim.x + (int)threadIdx.x; g < A.n_all;
+         g += ncta * (int)blockDim.x)
+      A.x[g] = A.x0[g];
+  while (ok && !T.done) {
+    double d[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      double2 zp[kRowSlots];
+#pragma unroll
+      for (int j = 0; j < kRowSlots; ++j) zp[j] = Q.load(at[k][j]);
+      double sum = 0.0;
+#pragma unroll
+      for (int j = 0; j < kRowSlots; ++j)
+        sum = dadd(sum, dmul(dadd(zp[j].x, dmul(T.beta, zp[j].y)), v[k][j]));
+      q[k] = sum;
+      p[k] = dadd(z[k], dmul(T.beta, p[k]));
+      d[0] = dadd(d[0], dmul(p[k], q[k]));  // (a thread without a row adds zeros)
+    }
+    if (!(ok = Q.template sum<1, false>(d))) break;
+    if (!alpha64(T, d[0], A.mode)) break;
+    double e[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = i0 + k * (int)blockDim.x;
+      r[k] = dadd(r[k], dmul(dmul(-1.0, T.alpha), q[k]));
+      z[k] = dadd(0.0, dmul(r[k], di[k]));
+      if (i < A.n) Q.publish(i, z[k], p[k]);
+      e[0] = dadd(e[0], dmul(r[k], z[k]));
+      e[1] = dadd(e[1], dmul(r[k], r[k]));
+      x[k] = dadd(x[k], dmul(T.alpha, p[k]));
+    }
+    if (!(ok = Q.template sum<2, true>(e))) break;
+    beta64(T, e, A.mode, A.maxit, A.tol);
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (i0 + k * (int)blockDim.x < A.n) A.x[i0 + k * (int)blockDim.x] = x[k];
+  if (!ok) T.status = GIPB200_ERR_TIMEOUT;
+  if (rank == 0 && threadIdx.x == 0) store64(A.S, T);
+}
+
+constexpr int kRegThreads = 256;  // CTA size of the register forms
+
+// Bound by latency: per iteration the gathers, the warp reductions and two cluster barriers.
+template <int K>
+__global__ void __launch_bounds__(kRegThreads, 1) k_pcg64_cluster(const __grid_constant__ Args64 A) {
+  __shared__ __align__(16) double2 pairs[K * kRegThreads];
+  __shared__ double red[2][3][8 * ClusterPairs::kMaxCtas];
+  ClusterPairs Q;
+  Q.rank = cluster_rank();
+  Q.size = cluster_size();
+  Q.rows = K * (int)blockDim.x;
+  Q.pairs = smem_u32(pairs);
+  Q.red = red;
+  cluster_barrier();  // every CTA runs before its shared memory is written
+  solve_rows<K>(A, Q, (int)Q.rank, (int)Q.size);
+  cluster_barrier();  // no CTA leaves while another may still read its pairs
+}
+
+template <int K>
+__global__ void __launch_bounds__(kRegThreads, 1) k_pcg64_grid(const __grid_constant__ Args64 A) {
+  GridPairs Q;
+  Q.pairs = A.pair;
+  Q.G = grid_begin(A.slots);
+  solve_rows<K>(A, Q, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// ------------------------------------------------------------------ streamed form
+// Several rows per thread: a CTA owns a contiguous range of slices; r and Ap (then z) of its
+// rows stay in shared memory, p, x and dinv in global memory, and the operator streams from
+// its packed layout (21 bytes a row) each iteration.  x += alpha p waits for the pass that
+// forms the next p, which reads p anyway.
+struct Stream64 {
+  const uint4* delta;
+  const void* idx;
+  const int* base;
+  const unsigned char* plain;
+  const double* table;
+  double* p;   // n_all entries, ghosts as x0 has them
+};
+
+// Operator words are read every iteration and meant to stay in L2.
+__device__ __forceinline__ uint4 ld_words(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned ld_word(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_word2(const uint2* p) {
+  uint2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+
+template <int NIB>
+__device__ __forceinline__ void words64(const Stream64& M, int s, int lane, PackedWords& w) {
+  const int i = s * 32 + lane;
+  w.plain = __ldg(M.plain + s);
+  w.d = ld_words(M.delta + i);
+  if (NIB == 4) {
+    w.w0 = ld_word(static_cast<const unsigned*>(M.idx) + i);
+    w.w1 = 0u;
+  } else {
+    const uint2 t = ld_word2(static_cast<const uint2*>(M.idx) + i);
+    w.w0 = t.x;
+    w.w1 = t.y;
+  }
+}
+
+// sum of row i of a sliced slice with plain loads of x (written inside the launch)
+__device__ __forceinline__ double row_plain(const SellView<double>& L, const double* x, int s,
+                                            int lane) {
+  long long base;
+  int len;
+  slice_range(L, s, base, len);
+  double sum = 0.0;
+  for (int j = 0; j < len; ++j) {
+    const int c = L.col[base + 32LL * j + lane];
+    if (c >= 0) sum = dadd(sum, dmul(x[c], L.val[base + 32LL * j + lane]));
+  }
+  return sum;
+}
+
+template <int NIB>
+__global__ void __launch_bounds__(1024, 1) k_pcg64_stream(const __grid_constant__ Args64 A,
+                                                          const __grid_constant__ Stream64 M) {
+  extern __shared__ __align__(16) double onchip[];
+  __shared__ double tab[NIB == 4 ? 16 : 256];
+  for (int t = threadIdx.x; t < (NIB == 4 ? 16 : 256); t += blockDim.x) tab[t] = M.table[t];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int rank = blockIdx.x, ncta = gridDim.x;
+  const int ns = A.L.nslices;
+  const int s0 = (int)((long long)ns * rank / ncta), s1 = (int)((long long)ns * (rank + 1) / ncta);
+  const int first = s0 * 32, rows = min(A.n, s1 * 32) - first;  // this CTA's rows
+  double* sr = onchip;                       // r
+  double* sq = onchip + (size_t)(s1 - s0) * 32;  // A p, then z
+  double* p = M.p;
+  GridScope G = grid_begin(A.slots);
+  double acc3[3] = {0.0, 0.0, 0.0};
+  for (int s = s0 + warp; s < s1; s += nw) {
+    const int i = s * 32 + lane;
+    const double sum = row_plain(A.L, A.x0, s, lane);
+    if (i < A.n) {
+      const double bi = A.b[i];
+      const double ri = dadd(bi, dmul(-1.0, sum));
+      const double zi = dadd(0.0, dmul(ri, A.dinv[i]));
+      sr[i - first] = ri;
+      p[i] = zi;
+      acc3[0] = dadd(acc3[0], dmul(ri, zi));
+      acc3[1] = dadd(acc3[1], dmul(ri, ri));
+      acc3[2] = dadd(acc3[2], dmul(bi, bi));
+    }
+  }
+  for (int g = A.n + rank * (int)blockDim.x + (int)threadIdx.x; g < A.n_all;
+       g += ncta * (int)blockDim.x)
+    p[g] = A.x0[g];
+  Scal64 T;
+  bool ok = grid_sum<3, true>(acc3, G);
+  start64(T, acc3, A.mode, A.maxit, A.tol);
+  if (A.x != A.x0) {  // (after the reduction: every row has read x0)
+    for (int k = threadIdx.x; k < rows; k += blockDim.x) A.x[first + k] = A.x0[first + k];
+    for (int g = A.n + rank * (int)blockDim.x + (int)threadIdx.x; g < A.n_all;
+         g += ncta * (int)blockDim.x)
+      A.x[g] = A.x0[g];
+  }
+  while (ok && !T.done) {
+    // A: Ap = L p, p.Ap
+    double d[1] = {0.0};
+    PackedWords w;
+    if (s0 + warp < s1) words64<NIB>(M, s0 + warp, lane, w);
+    for (int s = s0 + warp; s < s1; s += nw) {
+      const int i = s * 32 + lane;
+      PackedWords nx;
+      if (s + nw < s1) words64<NIB>(M, s + nw, lane, nx);
+      double sum = 0.0;
+      if (w.plain) {
+        sum = row_plain(A.L, p, s, lane);
+      } else {
+        int c[8];
+        packed_cols(M.base, s, w.d, c);
+        double xv[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) xv[j] = p[c[j]];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum = dadd(sum, dmul(xv[j], tab[packed_index<NIB>(w, j)]));
+      }
+      if (i < A.n) {
+        sq[i - first] = sum;
+        d[0] = dadd(d[0], dmul(p[i], sum));
+      }
+      w = nx;
+    }
+    if (!(ok = grid_sum<1, false>(d, G))) break;
+    if (!alpha64(T, d[0], A.mode)) break;
+    // B: r -= alpha Ap, z = dinv r (over Ap), r.z, r.r
+    const double malpha = dmul(-1.0, T.alpha);
+    double e[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int k = threadIdx.x; k < rows; k += 1024) {
+      const double ri = dadd(sr[k], dmul(malpha, sq[k]));
+      const double zi = dadd(0.0, dmul(ri, __ldg(A.dinv + first + k)));
+      sr[k] = ri;
+      sq[k] = zi;
+      e[0] = dadd(e[0], dmul(ri, zi));
+      e[1] = dadd(e[1], dmul(ri, ri));
+    }
+    if (!(ok = grid_sum<2, false>(e, G))) break;
+    beta64(T, e, A.mode, A.maxit, A.tol);
+    // C: x += alpha p; p = z + beta p (not after the last iteration)
+    if (T.done) {
+#pragma unroll 4
+      for (int k = threadIdx.x; k < rows; k += 1024)
+        A.x[first + k] = dadd(A.x[first + k], dmul(T.alpha, p[first + k]));
+      break;
+    }
+#pragma unroll 4
+    for (int k = threadIdx.x; k < rows; k += 1024) {
+      const double pk = p[first + k];
+      A.x[first + k] = dadd(A.x[first + k], dmul(T.alpha, pk));
+      p[first + k] = dadd(sq[k], dmul(T.beta, pk));
+    }
+    double none[1] = {0.0};
+    ok = grid_sum<1, true>(none, G);
+  }
+  if (!ok) T.status = GIPB200_ERR_TIMEOUT;
+  if (rank == 0 && threadIdx.x == 0) store64(A.S, T);
+}
+
+struct AlphaFinish64 {
+  PcgScalars* S;
+  int mode;
+  __device__ void operator()(const double* t) const {
+    S->pAp = t[0];
+    S->alpha = ddiv(S->rz, t[0]);
+    if (mode != GIPB200_PCG_FIXED && (!(t[0] > 0.0) || !isfinite(S->alpha))) {
+      S->status = GIPB200_ERR_BREAKDOWN;
+      S->done = 1;
+    }
+  }
+};
+
+// Ap = L p and p.Ap of the three-kernel loop (grids whose r and Ap do not fit on chip) from
+// the packed layout: 37 bytes a row instead of 100.
+template <int NIB>
+__global__ void __launch_bounds__(256, 8) k_pcg64_spmv_dot(SellView<double> L, Stream64 M,
+                                                           double* __restrict__ Ap, PcgScalars* S,
+                                                           ReduceScratch rs, int mode) {
+  if (S->done) return;
+  __shared__ double tab[NIB == 4 ? 16 : 256];
+  for (int t = threadIdx.x; t < (NIB == 4 ? 16 : 256); t += blockDim.x) tab[t] = M.table[t];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  const double* __restrict__ p = M.p;
+  double acc[1] = {0.0};
+  for (int s = gw; s < L.nslices; s += nw) {
+    PackedWords w;
+    packed_words<NIB>(M.delta, M.idx, M.plain, s, lane, w);
+    const int i = s * 32 + lane;
+    double sum = 0.0;
+    if (w.plain) {
+      sum = row_plain(L, p, s, lane);
+    } else {
+      int c[8];
+      packed_cols(M.base, s, w.d, c);
+#pragma unroll
+      for (int h = 0; h < 8; h += 4) {  // four gathers in flight at 32 registers
+        double xv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xv[j] = __ldg(p + c[h + j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum = dadd(sum, dmul(xv[j], tab[packed_index<NIB>(w, h + j)]));
+      }
+    }
+    if (i < L.nrows) {
+      Ap[i] = sum;
+      acc[0] = dadd(acc[0], dmul(p[i], sum));
+    }
+  }
+  grid_reduce<SumOp, 1>(acc, rs, AlphaFinish64{S, mode});
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ set-up
+// The packed layout of L in its stored slot order: eight 16-bit column deltas per row from a
+// base per (slice, slot) and eight indices into a table of L's values, as the mixed form
+// packs its FP32 operator (pcg.cu), but in GIP's order and in doubles.  Slots of ghost columns
+// (stored zeros) become padding.  Slices that do not fit keep the sliced layout.
+int Pcg::build_packed64(cudaStream_t s) {
+  const int ns = L->nslices;
+  const long long nslots = L->nslots;
+  if (ns == 0 || nslots == 0) return GIPB200_OK;
+  std::vector<long long> sptr((size_t)ns + 1);
+  std::vector<int> col((size_t)nslots);
+  std::vector<double> val((size_t)nslots);
+  GIPB_CUDA(cudaMemcpyAsync(sptr.data(), L->sptr.p, sptr.size() * 8, cudaMemcpyDeviceToHost, s));
+  GIPB_CUDA(cudaMemcpyAsync(col.data(), L->col.p, col.size() * 4, cudaMemcpyDeviceToHost, s));
+  GIPB_CUDA(cudaMemcpyAsync(val.data(), L->val.p, val.size() * 8, cudaMemcpyDeviceToHost, s));
+  GIPB_CUDA(cudaStreamSynchronize(s));
+  std::vector<double> tab;
+  if (!value_table(val.data(), nslots, 255, &tab)) return GIPB200_OK;
+  std::vector<unsigned long long> keys;
+  for (double t : tab)
+    if (t != 0.0 || std::signbit(t)) {
+      unsigned long long k;
+      memcpy(&k, &t, 8);
+      keys.push_back(k);
+    }
+  const int nib = keys.size() <= 15 ? 4 : 8;
+  std::vector<double> table((size_t)1 << nib, 0.0);
+  for (size_t t = 0; t < keys.size(); ++t) memcpy(&table[t + 1], &keys[t], 8);
+  const size_t rows = (size_t)ns * 32;
+  std::vector<uint4> delta(rows, make_uint4(0u, 0u, 0u, 0u));
+  std::vector<unsigned> idx4(nib == 4 ? rows : 0, 0u);
+  std::vector<uint2> idx8(nib == 8 ? rows : 0, make_uint2(0u, 0u));
+  std::vector<int> base((size_t)ns * 8, 0);
+  std::vector<unsigned char> plain((size_t)ns, 1);
+  long long packed = 0;
+  const int nu = n;
+#pragma omp parallel for schedule(static) reduction(+ : packed)
+  for (int sl = 0; sl < ns; ++sl) {
+    const long long b0 = sptr[sl];
+    const int len = (int)((sptr[sl + 1] - b0) >> 5);
+    if (len > 8) continue;
+    int lo[8], hi[8];
+    bool ok = true;
+    for (int j = 0; j < len && ok; ++j) {
+      lo[j] = 0x7fffffff;
+      hi[j] = -1;
+      for (int l = 0; l < 32; ++l) {
+        const int c = col[b0 + 32LL * j + l];
+        if (c < 0 || c >= nu) continue;
+        lo[j] = std::min(lo[j], c);
+        hi[j] = std::max(hi[j], c);
+      }
+      ok = hi[j] < 0 || hi[j] - lo[j] <= 65535;
+    }
+    if (!ok) continue;
+    plain[sl] = 0;
+    packed += 1;
+    for (int j = 0; j < len; ++j) base[(size_t)sl * 8 + j] = hi[j] >= 0 ? lo[j] : 0;
+    for (int l = 0; l < 32; ++l) {
+      unsigned dw[4] = {0u, 0u, 0u, 0u};
+      unsigned long long iw = 0ull;
+      for (int j = 0; j < len; ++j) {
+        const long long k = b0 + 32LL * j + l;
+        if (col[k] < 0 || col[k] >= nu) continue;
+        dw[j >> 1] |= (unsigned)(col[k] - lo[j]) << (16 * (j & 1));
+        unsigned long long bits;
+        memcpy(&bits, &val[k], 8);
+        if (bits == 0ull) continue;  // a stored +0.0: table entry 0
+        const unsigned t =
+            1u + (unsigned)(std::lower_bound(keys.begin(), keys.end(), bits) - keys.begin());
+        iw |= (unsigned long long)t << (nib * j);
+      }
+      const size_t r = (size_t)sl * 32 + l;
+      delta[r] = make_uint4(dw[0], dw[1], dw[2], dw[3]);
+      if (nib == 4) idx4[r] = (unsigned)iw;
+      else idx8[r] = make_uint2((unsigned)iw, (unsigned)(iw >> 32));
+    }
+  }
+  if (packed * 2 < ns) return GIPB200_OK;  // not worth a second layout
+  GIPB_TRY(op64.delta.upload(delta.data(), delta.size(), s));
+  if (nib == 4) GIPB_TRY(op64.idx4.upload(idx4.data(), idx4.size(), s));
+  else GIPB_TRY(op64.idx8.upload(idx8.data(), idx8.size(), s));
+  GIPB_TRY(op64.base.upload(base.data(), base.size(), s));
+  GIPB_TRY(op64.plain.upload(plain.data(), plain.size(), s));
+  GIPB_TRY(op64.table.upload(table.data(), table.size(), s));
+  GIPB_CUDA(cudaStreamSynchronize(s));
+  op64.bits = nib;
+  return GIPB200_OK;
+}
+
+namespace {
+
+size_t stream_shared(int nslices, int ncta) {
+  return (size_t)((nslices + ncta - 1) / ncta) * 32 * 2 * sizeof(double);
+}
+
+template <class K>
+bool stream_fits(K kern, size_t shared) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, kern) != cudaSuccess)
+    return false;
+  return shared + fa.sharedSizeBytes <= (size_t)most &&
+         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) ==
+             cudaSuccess;
+}
+
+template <class K>
+void one_launch_attr(K kern, const OneLaunch& o, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at,
+                     bool cluster) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3((unsigned)o.ctas);
+  cfg->blockDim = dim3((unsigned)o.threads);
+  cfg->dynamicSmemBytes = o.shared;
+  if (cluster) {
+    if (o.ctas > 8) (void)cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = (unsigned)o.ctas;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+  } else {
+    at->id = cudaLaunchAttributeCooperative;
+    at->val.cooperative = 1;
+  }
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+}
+
+template <class K>
+bool cluster_fits(K kern, const OneLaunch& o) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  one_launch_attr(kern, o, &cfg, at, true);
+  int most = 0;
+  if (cudaOccupancyMaxActiveClusters(&most, kern, &cfg) == cudaSuccess) return most >= 1;
+  (void)cudaGetLastError();
+  return false;
+}
+
+}  // namespace
+
+// Which one-launch form runs this solver's solves (FP64 modes with GIP's Jacobi).
+int Pcg::plan_one_launch(cudaStream_t s) {
+  one.form = OneLaunch::kNone;
+  if (prm.mode == GIPB200_PCG_MIXED || prm.precond != GIPB200_PRECOND_JACOBI || n <= 0 ||
+      !L->rows_nonempty || getenv("GIPB200_NO_ONE_LAUNCH"))
+    return GIPB200_OK;
+  int longest = 0;
+  for (int i = 0; i < n; ++i) longest = std::max(longest, L->h_rowptr[i + 1] - L->h_rowptr[i]);
+  bool ghosts_zero = true;  // the iterations drop ghost columns: all of them stored zeros
+  if (n_all > n) {
+    std::vector<double> hval((size_t)std::max(L->nnz, 1));
+    GIPB_CUDA(cudaMemcpyAsync(hval.data(), L->csr_val.p, (size_t)L->nnz * 8, cudaMemcpyDeviceToHost, s));
+    GIPB_CUDA(cudaStreamSynchronize(s));
+    for (int k = 0; k < L->nnz && ghosts_zero; ++k)
+      ghosts_zero = L->h_col[k] < n || hval[k] == 0.0;
+  }
+  if (!ghosts_zero) return GIPB200_OK;
+  DeviceInfo di;
+  GIPB_TRY(device_info(&di));
+  const int ctas = std::min(di.nsm, kGridCtasMax);
+  if (longest <= kRowSlots && n <= kRegThreads * 4 * ClusterPairs::kMaxCtas) {
+    // the fewest CTAs that leave a thread at most 4 rows, fewer rows while 8 CTAs (the
+    // portable cluster size) hold them
+    int k = n <= kRegThreads ? 1 : n <= kRegThreads * 2 * 8 ? 2 : 4;
+    int c = 1;
+    while (c * kRegThreads * k < n) c *= 2;
+    one.ctas = c;
+    one.per_thread = k;
+    one.threads = ((n + c * k - 1) / (c * k) + 31) / 32 * 32;
+    const bool fits = k == 1   ? cluster_fits(k_pcg64_cluster<1>, one)
+                      : k == 2 ? cluster_fits(k_pcg64_cluster<2>, one)
+                               : cluster_fits(k_pcg64_cluster<4>, one);
+    if (fits) {
+      one.form = OneLaunch::kCluster;
+      return GIPB200_OK;
+    }
+  }
+  if (longest <= kRowSlots && n <= kRegThreads * 4 * ctas) {
+    const int k = (n + kRegThreads * ctas - 1) / (kRegThreads * ctas);
+    one.form = OneLaunch::kGrid;
+    one.per_thread = k;
+    one.threads = kRegThreads;
+    one.ctas = (n + kRegThreads * k - 1) / (kRegThreads * k);
+    GIPB_TRY(one.pair.alloc((size_t)n));
+    return one.slots.alloc(grid_slot_count(one.ctas));
+  }
+  GIPB_TRY(build_packed64(s));
+  if (op64.bits) {
+    const size_t sh = stream_shared(L->nslices, ctas);
+    if (op64.bits == 4 ? stream_fits(k_pcg64_stream<4>, sh) : stream_fits(k_pcg64_stream<8>, sh)) {
+      one.form = OneLaunch::kStream;
+      one.threads = 1024;
+      one.ctas = ctas;
+      one.shared = sh;
+      return one.slots.alloc(grid_slot_count(ctas));
+    }
+  }
+  return GIPB200_OK;
+}
+
+namespace {
+template <class K, class... Args>
+int launch_one(K kern, const OneLaunch& o, cudaStream_t s, const Args&... args) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[1];
+  one_launch_attr(kern, o, &cfg, at, o.form == OneLaunch::kCluster);
+  cfg.stream = s;
+  GIPB_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  return GIPB200_OK;
+}
+}  // namespace
+
+static Stream64 stream64(const Pcg& P) {
+  const Packed64& o = P.op64;
+  return {o.delta.p, o.bits == 4 ? (const void*)o.idx4.p : (const void*)o.idx8.p, o.base.p,
+          o.plain.p, o.table.p, P.p.p};
+}
+
+int Pcg::enqueue_one_launch(const double* b, double* x, const double* x0, cudaStream_t s) {
+  Args64 A{L->view(), b, x0, dinv.p, x, one.pair.p, one.slots.p, sc.p, prm.tol, n, n_all,
+           prm.mode, prm.maxit};
+  launches += 1;
+  if (one.form != OneLaunch::kCluster)
+    GIPB_CUDA(cudaMemsetAsync(one.slots.p, 0, one.slots.n * sizeof(ulonglong2), s));
+  const int k = one.per_thread;
+  switch (one.form) {
+    case OneLaunch::kCluster:
+      return k == 1   ? launch_one(k_pcg64_cluster<1>, one, s, A)
+             : k == 2 ? launch_one(k_pcg64_cluster<2>, one, s, A)
+                      : launch_one(k_pcg64_cluster<4>, one, s, A);
+    case OneLaunch::kGrid:
+      return k == 1   ? launch_one(k_pcg64_grid<1>, one, s, A)
+             : k == 2 ? launch_one(k_pcg64_grid<2>, one, s, A)
+             : k == 3 ? launch_one(k_pcg64_grid<3>, one, s, A)
+                      : launch_one(k_pcg64_grid<4>, one, s, A);
+    default: {
+      const Stream64 M = stream64(*this);
+      return op64.bits == 4 ? launch_one(k_pcg64_stream<4>, one, s, A, M)
+                            : launch_one(k_pcg64_stream<8>, one, s, A, M);
+    }
+  }
+}
+
+void Pcg::launch_packed64_spmv(double* q, PcgScalars* S, int mode, cudaStream_t s) {
+  const Stream64 M = stream64(*this);
+  if (op64.bits == 4)
+    k_pcg64_spmv_dot<4><<<blocks_spmv, 256, 0, s>>>(L->view(), M, q, S, rs, mode);
+  else
+    k_pcg64_spmv_dot<8><<<blocks_spmv, 256, 0, s>>>(L->view(), M, q, S, rs, mode);
+}
+
+}  // namespace gipb200

@@ -1,0 +1,142 @@
+"""FP64 Jacobi-PCG as one launch: the cluster, grid and streamed forms at the edges of their
+ranges, against the oracle's GIP_LinearSolver."""
+import numpy as np
+import pytest
+import torch
+
+from gip_b200.formats import Csr
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _band(n, n_all, far=0, values=0, seed=0, ghost=0.0):
+    """SPD band matrix: couplings to i +- 1, i +- 37 and (far > 0) of every far-th row to a
+    row across the matrix; `values` > 0 draws the diagonal from that many doubles.  Columns
+    past n (ghosts) hold `ghost`."""
+    rng = np.random.default_rng(seed)
+    i = np.arange(n)
+    rows, cols, vals = [], [], []
+    for d in (1, 37):
+        a = i[:-d] if d < n else i[:0]
+        rows += [a, a + d]
+        cols += [a + d, a]
+        vals += [np.full(a.size, -1.0)] * 2
+    if far:
+        a = i[: n // 2 : far]
+        b = a + n // 2
+        rows += [a, b]
+        cols += [b, a]
+        vals += [np.full(a.size, -0.5)] * 2
+    if n_all > n:
+        g = np.arange(min(n_all - n, n))
+        rows.append(g)
+        cols.append(n + g)
+        vals.append(np.full(g.size, ghost))
+    diag = 6.5 + (rng.integers(0, values, n) / 16.0 if values else 0.0) * np.ones(n)
+    rows.append(i)
+    cols.append(i)
+    vals.append(diag)
+    r, c, v = np.concatenate(rows), np.concatenate(cols), np.concatenate(vals)
+    o = np.lexsort((c, r))
+    r, c, v = r[o], c[o], v[o]
+    rp = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(r, minlength=n), out=rp[1:])
+    return Csr(n, n_all, rp.astype(np.int32), c.astype(np.int32), v.astype(np.float64))
+
+
+def _close(got, want):
+    """Within 1e-10 of the scale; NaN where the oracle has NaN (one unknown is solved after
+    one iteration, and GIP's fixed iterations then divide 0 by 0)."""
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    fine = ~np.isnan(want)
+    if fine.any():
+        assert np.abs(got - want)[fine].max() <= 1e-10 * np.abs(want[fine]).max()
+
+
+SIZES = [1, 31, 32, 33, 256, 257, 4096, 4097, 16384, 16385, 37888, 37889, 151552, 151553]
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_forms_match_oracle_at_their_edges(gpu, oracle_mod, n):
+    # fixed iterations from a nonzero start with zero-valued ghost columns; the solver's
+    # parity bar (1e-10 of the solution's scale) as for the three-kernel loop
+    from gip_b200 import device as dv
+    n_all = n + min(n, 40)
+    L = _band(n, n_all, far=1000, seed=n)
+    rng = np.random.default_rng(n)
+    b, x0 = rng.standard_normal(n), rng.standard_normal(n_all)
+    xr, it, _ = oracle_mod.pcg(L, b, x0, maxit=9, mode=0)
+    S = dv.PcgSolver(dv.DeviceMatrix(L), n_all=n_all, mode="fixed", maxit=9)
+    x = _t(np.zeros(n_all))
+    for start in (_t(x0), None):   # a separate start, then x = x0 in place
+        if start is None:
+            x.copy_(_t(x0))
+        res = S.solve(_t(b), x, x if start is None else start)
+        assert res["iterations"] == it == 9
+        got = x.cpu().numpy()
+        assert np.array_equal(got[n:], x0[n:])
+        _close(got, xr)
+
+
+@pytest.mark.parametrize("n,far,values", [(151600, 32, 0), (160001, 5000, 100), (160001, 0, 300),
+                                          (2300001, 0, 0)])
+def test_streamed_form_layouts(gpu, oracle_mod, n, far, values):
+    # packed rows beside plain slices (far couplings spread a slot over more than 16 bits), an
+    # 8-bit value table, an operator without a table (three kernels), and more rows than the
+    # shared memory holds (three kernels on the packed operator)
+    from gip_b200 import device as dv
+    L = _band(n, n, far=far, values=values, seed=3)
+    b = np.random.default_rng(5).standard_normal(n)
+    xr, it, rr = oracle_mod.pcg(L, b, np.zeros(n), maxit=500, mode=1, tol=1e-9)
+    S = dv.PcgSolver(dv.DeviceMatrix(L), mode="tol", maxit=500, tol=1e-9)
+    x = _t(np.zeros(n))
+    res = S.solve(_t(b), x, _t(np.zeros(n)))
+    assert res["status"] == 0 and abs(res["iterations"] - it) <= 1
+    if res["iterations"] == it:
+        _close(x.cpu().numpy(), xr)
+
+
+@pytest.mark.parametrize("n", [100, 5000, 20000, 152000])
+def test_forms_follow_the_general_path(gpu, monkeypatch, n):
+    # failures and special starts come out as the three-kernel loop has them
+    from gip_b200 import device as dv
+    L = _band(n, n + 8, seed=1)
+    A = dv.DeviceMatrix(L)
+    rng = np.random.default_rng(2)
+    b, x0 = rng.standard_normal(n), rng.standard_normal(n + 8)
+    bad = b.copy()
+    bad[n // 3] = np.nan
+    inf = x0.copy()
+    inf[n + 3] = np.inf          # a ghost entry: its stored zero makes the residual NaN
+    out = []
+    for general in (False, True):
+        if general:
+            monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+        got = []
+        for mode, maxit, rhs, start in (("tol", 2, b, x0), ("tol", 50, bad, x0), ("tol", 50, b, inf),
+                                        ("fixed", 3, bad, x0), ("tol", 50, np.zeros(n), 0 * x0),
+                                        ("fixed", 0, b, x0)):
+            S = dv.PcgSolver(A, n_all=n + 8, mode=mode, maxit=maxit, tol=1e-9)
+            x = _t(np.ones(n + 8))
+            r = S.solve(_t(rhs), x, _t(start))
+            got.append((r["status"], r["iterations"], bool(torch.isfinite(x[:n]).all())))
+        out.append(got)
+    assert out[0] == out[1], out
+
+
+def test_nonzero_ghost_values_keep_the_general_path(gpu, oracle_mod):
+    # ghost columns with nonzero values read the start's ghost entries in every product
+    from gip_b200 import device as dv
+    n = 300
+    L = _band(n, n + 20, seed=4, ghost=-0.25)
+    rng = np.random.default_rng(6)
+    b, x0 = rng.standard_normal(n), rng.standard_normal(n + 20)
+    xr, it, _ = oracle_mod.pcg(L, b, x0, maxit=9, mode=0)
+    S = dv.PcgSolver(dv.DeviceMatrix(L), n_all=n + 20, mode="fixed", maxit=9)
+    x = _t(np.zeros(n + 20))
+    S.solve(_t(b), x, _t(x0))
+    _close(x.cpu().numpy(), xr)
