@@ -36,9 +36,9 @@ void setup_mark(const char* what) {
   last = now;
 }
 
-bool pdl_enabled() {
-  const char* e = getenv("GIPB200_PDL");  // read at each launch (captured graphs keep it)
-  return e && e[0] == '1';
+bool dependent_launches(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
 }
 
 // ------------------------------------------------------------------ device info
