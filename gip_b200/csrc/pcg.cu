@@ -938,8 +938,8 @@ int Pcg::init(const Sell* Lm, int nall, const gipb200_pcg_params& params, cudaSt
       GIPB_CUDA(cudaStreamSynchronize(s));
     }
     if (prm.precond == GIPB200_PRECOND_AMG) GIPB_TRY(build_amg64(s));
-    GIPB_TRY(plan_one_launch(s));
   }
+  GIPB_TRY(plan_one_launch(s));
   GIPB_CUDA(cudaStreamSynchronize(s));
   return GIPB200_OK;
 }
@@ -1465,7 +1465,9 @@ int Pcg::enqueue_mixed_graph(const double* b, double* x, const double* x0, cudaS
   if (x != x0) GIPB_CUDA(cudaMemcpyAsync(x, x0, (size_t)n_all * 8, cudaMemcpyDeviceToDevice, s));
   GIPB_CUDA(cudaMemsetAsync(sc.p, 0, sizeof(PcgScalars), s));
   if (amg) GIPB_TRY(amg->reset_tail(s));
-  GIPB_TRY(launch_mixed_residual(b, x, 1, s, 1, hl));
+  const double* bp = b;
+  if (lpacked) GIPB_TRY(enqueue_ghost_rhs(b, x, s, &bp));
+  GIPB_TRY(launch_mixed_residual(b, bp, x, 1, s, 1, hl));
   if (amg) GIPB_TRY(amg->enqueue(a32(), r32.p, z32.p, sc.p, rs, 0, s, &pk0));
   cudaGraph_t loop_body;
   GIPB_TRY(add_while(s, hl, &loop_body));
@@ -1494,7 +1496,7 @@ int Pcg::enqueue_mixed_graph(const double* b, double* x, const double* x0, cudaS
       GIPB_CUDA(cudaStreamBeginCaptureToGraph(is, if_body, nullptr, nullptr, 0,
                                               cudaStreamCaptureModeRelaxed));
       launch_dep(k_mx_apply, blocks_vec, 256, is, n, x, y32.p, (const double*)scale.p, sc.p);
-      int rst = launch_mixed_residual(b, x, 0, is, 0, 0);
+      int rst = launch_mixed_residual(b, bp, x, 0, is, 0, 0);
       cudaError_t le = cudaGetLastError();
       cudaGraph_t out = nullptr;
       GIPB_CUDA(cudaStreamEndCapture(is, &out));
@@ -1580,25 +1582,29 @@ static void launch_mx_spmv(const Pcg& P, const float* pin, float* pout, const fl
 #undef GIPB_MXP
 }
 
-int Pcg::launch_mixed_residual(const double* b, const double* x, int first, cudaStream_t s,
-                               int use_cond, cudaGraphConditionalHandle h) {
+int Pcg::enqueue_ghost_rhs(const double* b, const double* x, cudaStream_t s, const double** bp) {
+  const int ng = (int)ghost_rows.size();
+  *bp = b;
+  if (ng == 0) return GIPB200_OK;
+  GIPB_CUDA(cudaMemcpyAsync(bprime.p, b, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  int gb = 1;
+  GIPB_TRY(grid_blocks(256, ng, 1, 0, &gb));
+  k_mx_ghost_rhs<<<gb, 256, 0, s>>>(ng, d_ghost_rows.p, d_ghost_rp.p, d_ghost_col.p,
+                                    d_ghost_val.p, x, b, bprime.p);
+  GIPB_LAUNCH_CHECK();
+  launches += 1;
+  *bp = bprime.p;
+  return GIPB200_OK;
+}
+
+// bp: b less L's ghost part for this solve (x's ghost entries stay fixed during a solve)
+int Pcg::launch_mixed_residual(const double* b, const double* bp, const double* x, int first,
+                               cudaStream_t s, int use_cond, cudaGraphConditionalHandle h) {
   if (lpacked) {
-    if (first) {  // b' = b - L_ghost x for this solve (x's ghost entries stay fixed)
-      GIPB_CUDA(cudaMemcpyAsync(bprime.p, b, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice,
-                                s));
-      const int ng = (int)ghost_rows.size();
-      if (ng > 0) {
-        int gb = 1;
-        GIPB_TRY(grid_blocks(256, ng, 1, 0, &gb));
-        k_mx_ghost_rhs<<<gb, 256, 0, s>>>(ng, d_ghost_rows.p, d_ghost_rp.p, d_ghost_col.p,
-                                          d_ghost_val.p, x, b, bprime.p);
-        launches += 1;
-      }
-    }
     launch_dep(k_mx_residual_packed, blocks_spmv, 256, s, L->view(),
                (const uint4*)cop.delta.p, (const int*)cop.base.p,
                (const unsigned char*)cop.plain.p, (const unsigned*)lidx4.p,
-               (const double*)ltable.p, (const double*)bprime.p, (const double*)x, b,
+               (const double*)ltable.p, bp, (const double*)x, b,
                (const double*)scale.p, r32.p, p32.p, y32.p, sc.p, rs, first, prm.tol,
                prm.inner_tol, prm.maxit, prm.max_outer, pin_row, pin_val, use_cond, h,
                amg ? 1 : 0);
@@ -1620,7 +1626,9 @@ int Pcg::enqueue_mixed(const double* b, double* x, const double* x0, cudaStream_
   if (x != x0) GIPB_CUDA(cudaMemcpyAsync(x, x0, (size_t)n_all * 8, cudaMemcpyDeviceToDevice, s));
   GIPB_CUDA(cudaMemsetAsync(sc.p, 0, sizeof(PcgScalars), s));
   if (amg) GIPB_TRY(amg->reset_tail(s));
-  GIPB_TRY(launch_mixed_residual(b, x, 1, s, 0, 0));
+  const double* bp = b;
+  if (lpacked) GIPB_TRY(enqueue_ghost_rhs(b, x, s, &bp));
+  GIPB_TRY(launch_mixed_residual(b, bp, x, 1, s, 0, 0));
   if (amg) GIPB_TRY(amg->enqueue(a32(), r32.p, z32.p, sc.p, rs, 0, s, &pk0));
   const int poll = host_poll_interval();
   for (int k = 0; k < prm.maxit; ++k) {
@@ -1634,7 +1642,7 @@ int Pcg::enqueue_mixed(const double* b, double* x, const double* x0, cudaStream_
                (const double*)scale.p, 0, (cudaGraphConditionalHandle)0, amg ? 1 : 0);
     launch_dep(k_mx_apply, blocks_vec, 256, s, n, x, y32.p, (const double*)scale.p, sc.p);
     GIPB_LAUNCH_CHECK();
-    GIPB_TRY(launch_mixed_residual(b, x, 0, s, 0, 0));
+    GIPB_TRY(launch_mixed_residual(b, bp, x, 0, s, 0, 0));
     if (amg) GIPB_TRY(amg->enqueue(a32(), r32.p, z32.p, sc.p, rs, 0, s, &pk0));
     launches += 4;
     if (host_sync && (k + 1) % poll == 0) {

@@ -59,6 +59,7 @@ struct CompressedOp {
 // The FP64 operator packed in GIP's slot order (build_packed64); bits = 0: not built.
 struct Packed64 {
   int bits = 0;                  // value-table index bits: 4 or 8
+  int slots = 8;                 // 7: no packed row uses the eighth slot
   DevBuf<uint4> delta;
   DevBuf<unsigned> idx4;
   DevBuf<uint2> idx8;
@@ -67,14 +68,20 @@ struct Packed64 {
   DevBuf<double> table;
 };
 
-// How a whole FP64 Jacobi solve runs as one launch (persist.cu); kNone: kernel by kernel.
+// How a whole solve runs as one launch; kNone: kernel by kernel.  kCluster, kGrid, kStream:
+// FP64 with GIP's Jacobi (persist.cu); kSolve: the mixed form and the FP64 tolerance mode
+// with AMG (persist_amg.cu).
 struct OneLaunch {
-  enum { kNone = 0, kCluster, kGrid, kStream };
+  enum { kNone = 0, kCluster, kGrid, kStream, kSolve };
   int form = kNone;
   int ctas = 0, threads = 0;
   int per_thread = 1;            // register forms: rows per thread
   size_t shared = 0;             // dynamic shared memory per CTA
-  DevBuf<double2> pair;          // kGrid: (z, p) of every row
+  DevBuf<double2> pair;          // kGrid, kSolve: (z, p) of every row
+  DevBuf<unsigned char> ops;     // kSolve: the V-cycle's products
+  int nops = 0;
+  DevBuf<double> rd;             // kSolve, mixed: the FP64 residual and partial sums of it
+  bool cluster = false;          // kSolve: over a cluster instead of a cooperative grid
   DevBuf<ulonglong2> slots;      // grid reductions
 };
 
@@ -148,7 +155,13 @@ struct Pcg {
   // several solvers advance side by side on one GPU (a batch): forms that claim every SM at
   // once (the cooperative ones) would take turns, so only the cluster form runs
   bool shared_gpu = false;
+  // a step history counts the kernels of every solve against its iterations: the mixed form
+  // with Jacobi and the FP64 form with AMG of an engine keep their kernels
+  bool counted = false;
   bool one_launch() const {
+    if (one.form == OneLaunch::kSolve && counted &&
+        (prm.mode == GIPB200_PCG_MIXED) != (prm.precond == GIPB200_PRECOND_AMG))
+      return false;
     return one.form == OneLaunch::kCluster || (one.form != OneLaunch::kNone && !shared_gpu);
   }
   // scalars and reduction scratch
@@ -184,6 +197,11 @@ struct Pcg {
  private:
   int build_packed64(cudaStream_t s);
   int plan_one_launch(cudaStream_t s);
+  int plan_solve_launch(cudaStream_t s);
+  int enqueue_solve_launch(const double* b, double* x, const double* x0, cudaStream_t s);
+  int ghosts_zero(cudaStream_t s, bool* zero) const;  // L's ghost columns all hold 0.0
+  // b less L's ghost part into bprime (*bp: bprime, or b itself without ghost rows)
+  int enqueue_ghost_rhs(const double* b, const double* x, cudaStream_t s, const double** bp);
   void launch_packed64_spmv(double* q, PcgScalars* S, int mode, cudaStream_t s);
   // operator bytes a product streams from the packed FP64 layout: column deltas, value
   // indices, the slices' slot bases
@@ -195,7 +213,8 @@ struct Pcg {
   int read_flag(cudaStream_t s, int which, int* v);
   int enqueue_fp64_graph(const double* b, double* x, const double* x0, cudaStream_t s);
   int enqueue_mixed_graph(const double* b, double* x, const double* x0, cudaStream_t s);
-  int launch_mixed_residual(const double* b, const double* x, int first, cudaStream_t s,
+  int launch_mixed_residual(const double* b, const double* bp, const double* x, int first,
+                            cudaStream_t s,
                             int use_cond, cudaGraphConditionalHandle h);
 };
 

@@ -547,8 +547,9 @@ int Pcg::build_packed64(cudaStream_t s) {
   std::vector<int> base((size_t)ns * 8, 0);
   std::vector<unsigned char> plain((size_t)ns, 1);
   long long packed = 0;
+  int longest = 0;
   const int nu = n;
-#pragma omp parallel for schedule(static) reduction(+ : packed)
+#pragma omp parallel for schedule(static) reduction(+ : packed) reduction(max : longest)
   for (int sl = 0; sl < ns; ++sl) {
     const long long b0 = sptr[sl];
     const int len = (int)((sptr[sl + 1] - b0) >> 5);
@@ -569,6 +570,7 @@ int Pcg::build_packed64(cudaStream_t s) {
     if (!ok) continue;
     plain[sl] = 0;
     packed += 1;
+    longest = std::max(longest, len);
     for (int j = 0; j < len; ++j) base[(size_t)sl * 8 + j] = hi[j] >= 0 ? lo[j] : 0;
     for (int l = 0; l < 32; ++l) {
       unsigned dw[4] = {0u, 0u, 0u, 0u};
@@ -599,6 +601,7 @@ int Pcg::build_packed64(cudaStream_t s) {
   GIPB_TRY(op64.table.upload(table.data(), table.size(), s));
   GIPB_CUDA(cudaStreamSynchronize(s));
   op64.bits = nib;
+  op64.slots = longest <= 7 ? 7 : 8;
   return GIPB200_OK;
 }
 
@@ -655,23 +658,27 @@ bool cluster_fits(K kern, const OneLaunch& o) {
 
 }  // namespace
 
-// Which one-launch form runs this solver's solves (FP64 modes with GIP's Jacobi).
+int Pcg::ghosts_zero(cudaStream_t s, bool* zero) const {
+  *zero = true;
+  if (n_all <= n) return GIPB200_OK;
+  std::vector<double> hval((size_t)std::max(L->nnz, 1));
+  GIPB_CUDA(cudaMemcpyAsync(hval.data(), L->csr_val.p, (size_t)L->nnz * 8, cudaMemcpyDeviceToHost, s));
+  GIPB_CUDA(cudaStreamSynchronize(s));
+  for (int k = 0; k < L->nnz && *zero; ++k) *zero = L->h_col[k] < n || hval[k] == 0.0;
+  return GIPB200_OK;
+}
+
+// Which one-launch form runs this solver's solves.
 int Pcg::plan_one_launch(cudaStream_t s) {
   one.form = OneLaunch::kNone;
-  if (prm.mode == GIPB200_PCG_MIXED || prm.precond != GIPB200_PRECOND_JACOBI || n <= 0 ||
-      !L->rows_nonempty || getenv("GIPB200_NO_ONE_LAUNCH"))
-    return GIPB200_OK;
+  if (prm.mode == GIPB200_PCG_MIXED || prm.precond != GIPB200_PRECOND_JACOBI)
+    return plan_solve_launch(s);
+  if (n <= 0 || !L->rows_nonempty || getenv("GIPB200_NO_ONE_LAUNCH")) return GIPB200_OK;
   int longest = 0;
   for (int i = 0; i < n; ++i) longest = std::max(longest, L->h_rowptr[i + 1] - L->h_rowptr[i]);
-  bool ghosts_zero = true;  // the iterations drop ghost columns: all of them stored zeros
-  if (n_all > n) {
-    std::vector<double> hval((size_t)std::max(L->nnz, 1));
-    GIPB_CUDA(cudaMemcpyAsync(hval.data(), L->csr_val.p, (size_t)L->nnz * 8, cudaMemcpyDeviceToHost, s));
-    GIPB_CUDA(cudaStreamSynchronize(s));
-    for (int k = 0; k < L->nnz && ghosts_zero; ++k)
-      ghosts_zero = L->h_col[k] < n || hval[k] == 0.0;
-  }
-  if (!ghosts_zero) return GIPB200_OK;
+  bool zero = true;  // the iterations drop ghost columns: all of them stored zeros
+  GIPB_TRY(ghosts_zero(s, &zero));
+  if (!zero) return GIPB200_OK;
   DeviceInfo di;
   GIPB_TRY(device_info(&di));
   const int ctas = std::min(di.nsm, kGridCtasMax);
@@ -734,6 +741,7 @@ static Stream64 stream64(const Pcg& P) {
 }
 
 int Pcg::enqueue_one_launch(const double* b, double* x, const double* x0, cudaStream_t s) {
+  if (one.form == OneLaunch::kSolve) return enqueue_solve_launch(b, x, x0, s);
   Args64 A{L->view(), b, x0, dinv.p, x, one.pair.p, one.slots.p, sc.p, prm.tol, n, n_all,
            prm.mode, prm.maxit};
   launches += 1;

@@ -10,7 +10,7 @@ namespace gipb200 {
 
 // A grid wait that would never end gives up after about 2 s of SM clock.
 constexpr long long kGridSpinCycles = 4000000000LL;
-constexpr int kGridSums = 4;       // sums per grid reduction
+constexpr int kGridSums = 5;       // sums per grid reduction
 constexpr int kGridCtasMax = 256;  // CTAs of a grid reduction (each polled by one thread)
 // 16-byte slots of one grid's reductions: [2 parities][kGridSums][CTA], then the arrival
 // counter; all zero at launch
@@ -53,10 +53,12 @@ struct GridScope {
   bool ok;  // false: a wait gave up (the same in every thread after the call that noticed)
 };
 
-__device__ __forceinline__ GridScope grid_begin(ulonglong2* slots) {
-  const int ncta = (int)gridDim.x;
+__device__ __forceinline__ GridScope grid_begin(ulonglong2* slots, int rank, int ncta) {
   return GridScope{slots, reinterpret_cast<unsigned*>(slots + (size_t)2 * kGridSums * ncta), 0u,
-                   ncta, (int)blockIdx.x, true};
+                   ncta, rank, true};
+}
+__device__ __forceinline__ GridScope grid_begin(ulonglong2* slots) {
+  return grid_begin(slots, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // FENCE: the reduction is also a barrier for global memory (what any thread of the grid wrote
@@ -134,6 +136,38 @@ __device__ __forceinline__ bool grid_sum(double (&v)[W], GridScope& G) {
     for (int i = 1; i < nwait; ++i) a = dadd(a, sh2[k][i]);
     v[k] = a;
   }
+  if (s_fail) G.ok = false;
+  return G.ok;
+}
+
+// A grid barrier in two halves: between them a CTA may load what no CTA of the grid writes.
+__device__ __forceinline__ void grid_arrive(GridScope& G) {
+  G.epoch += 1u;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(G.count) : "memory");
+  }
+}
+// Every thread of the grid has arrived and what it wrote before is visible; false: gave up.
+__device__ __forceinline__ bool grid_wait(GridScope& G) {
+  __shared__ int s_fail;
+  if (threadIdx.x == 0) {
+    const unsigned target = G.epoch * (unsigned)G.ncta;
+    const long long t0 = clock64();
+    unsigned c;
+    s_fail = 0;
+    while (true) {
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(G.count) : "memory");
+      if ((int)(c - target) >= 0) break;
+      if (clock64() - t0 > kGridSpinCycles) {
+        s_fail = 1;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
   if (s_fail) G.ok = false;
   return G.ok;
 }

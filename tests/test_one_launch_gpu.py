@@ -140,3 +140,85 @@ def test_nonzero_ghost_values_keep_the_general_path(gpu, oracle_mod):
     x = _t(np.zeros(n + 20))
     S.solve(_t(b), x, _t(x0))
     _close(x.cpu().numpy(), xr)
+
+
+SOLVES = {
+    "mixed": dict(mode="mixed", maxit=5000, tol=1e-10, inner_tol=0.1, max_outer=100),
+    "mixed_amg": dict(mode="mixed", maxit=2000, tol=1e-10, inner_tol=1e-2, max_outer=100,
+                      precond="amg"),
+    "tol_amg": dict(mode="tol", maxit=2000, tol=1e-10, precond="amg"),
+}
+
+
+@pytest.mark.parametrize("solve", sorted(SOLVES))
+@pytest.mark.parametrize("n", [11, 16, 17, 27, 28, 40])
+def test_preconditioned_solves_as_one_launch(gpu, monkeypatch, solve, n):
+    # clusters of 8 (to 4096 rows) and 16 (to 20000) and the cooperative grid, on the cavity's
+    # pinned operator with ghost columns from a nonzero start, against the same solver kernel
+    # by kernel: the same row sums, dots added in another order, so the iterates agree far
+    # below the tolerance's own error (conditioning x 1e-10)
+    from gip_b200 import cavity
+    from gip_b200 import device as dv
+    case, _ = cavity.generate(n, re=100.0)
+    L = case.ops["L"]
+    A = dv.DeviceMatrix(L)
+    rng = np.random.default_rng(n)
+    b, x0 = rng.standard_normal(L.nrows), rng.standard_normal(case.n_owned) * 0.1
+    S = dv.PcgSolver(A, n_all=case.n_owned, **SOLVES[solve])
+    monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+    K = dv.PcgSolver(A, n_all=case.n_owned, **SOLVES[solve])
+    xs, xk = _t(np.zeros(case.n_owned)), _t(np.zeros(case.n_owned))
+    rk = K.solve(_t(b), xk, _t(x0))
+    for alias in (False, True):
+        if alias:
+            xs.copy_(_t(x0))
+        rs = S.solve(_t(b), xs, xs if alias else _t(x0))
+        assert rs["status"] == rk["status"] == 0
+        assert abs(rs["iterations"] - rk["iterations"]) <= 0.1 * rk["iterations"] + 1
+        got, want = xs.cpu().numpy(), xk.cpu().numpy()
+        assert np.array_equal(got[L.nrows:], x0[L.nrows:])
+        assert np.abs(got - want).max() <= 1e-8 * np.abs(want).max()
+        r = b - L.to_scipy() @ got
+        assert np.linalg.norm(r) <= 1.0001e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("solve", sorted(SOLVES))
+def test_preconditioned_one_launch_statuses(gpu, monkeypatch, solve):
+    from gip_b200 import cavity
+    from gip_b200 import device as dv
+    L, b = cavity.poisson_problem(14, seed=2)
+    A = dv.DeviceMatrix(L)
+    bad = b.copy()
+    bad[17] = np.nan
+    out = []
+    for general in (False, True):
+        if general:
+            monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+        S = dv.PcgSolver(A, **SOLVES[solve])
+        T = dv.PcgSolver(A, **dict(SOLVES[solve], maxit=2))
+        got = []
+        for slv, rhs in ((S, bad), (S, b), (T, b), (S, 0 * b)):
+            x = _t(np.ones(L.nrows))
+            r = slv.solve(_t(rhs), x, _t(np.zeros(L.nrows)))
+            got.append((r["status"], bool(torch.isfinite(x).all())))
+        out.append(got)
+    assert out[0] == out[1] and out[0][1][0] == 0, out
+
+
+@pytest.mark.parametrize("values,far", [(0, 32), (100, 700), (300, 0)])
+def test_preconditioned_one_launch_layouts(gpu, monkeypatch, values, far):
+    # plain slices beside packed ones, an 8-bit value table, and an operator that does not
+    # pack: the same solutions kernel by kernel
+    from gip_b200 import device as dv
+    n = 70000
+    A = dv.DeviceMatrix(_band(n, n, far=far, values=values, seed=8))
+    b = np.random.default_rng(3).standard_normal(n)
+    for solve in sorted(SOLVES):
+        monkeypatch.delenv("GIPB200_NO_ONE_LAUNCH", raising=False)
+        S = dv.PcgSolver(A, **SOLVES[solve])
+        monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+        K = dv.PcgSolver(A, **SOLVES[solve])
+        xs, xk = _t(np.zeros(n)), _t(np.zeros(n))
+        rs, rk = S.solve(_t(b), xs, _t(np.zeros(n))), K.solve(_t(b), xk, _t(np.zeros(n)))
+        assert rs["status"] == rk["status"] == 0, (solve, rs, rk)
+        assert float((xs - xk).abs().max()) <= 1e-8 * float(xk.abs().max()), solve
