@@ -175,6 +175,7 @@ struct Sell {
   int nrows = 0, ncols = 0, nnz = 0, nslices = 0;
   long long nslots = 0;
   bool rows_nonempty = true;  // no empty row
+  unsigned version = 0;       // counts changes of the values (layouts packed from them lapse)
   int uslots = 0;             // > 0: every slice has this many slots
   DevBuf<long long> sptr;
   DevBuf<int> col;
@@ -220,6 +221,27 @@ bool value_table(const double* v, long long n, int cap, std::vector<double>* tab
 int validate_csr(int nrows, int ncols, int nnz, const int* rowptr, const int* col,
                  int col_bound, const char* name);
 
+// An FP64 operator compressed without loss, in its stored slot order (bits = 0: not built).  A
+// slice of 32 rows whose rows have at most 8 slots and whose column spread per slot fits 16
+// bits is packed per row: eight 16-bit column deltas (one 16-byte load) from a per-(slice,
+// slot) base, and eight indices into a table of the operator's at most 255 distinct values (4
+// bits when there are at most 15; index 0 = padding).  Other slices stay sliced.
+struct Packed64 {
+  int bits = 0;                  // value-table index bits: 4 or 8
+  int slots = 8;                 // 7: no packed row uses the eighth slot
+  DevBuf<uint4> delta;           // per row (nslices * 32)
+  DevBuf<unsigned> idx4;         // per row, 8 x 4 bits
+  DevBuf<uint2> idx8;            // per row, 8 x 8 bits
+  DevBuf<int> base;              // per slice, 8 slots
+  DevBuf<unsigned char> plain;   // per slice
+  DevBuf<double> table;          // 16 or 256 entries
+};
+int pack64(const Sell& S, int cols, bool keep_zeros, Packed64* out, cudaStream_t s);
+int launch_packed_spmv(const Sell& A, const Packed64& P, const double* x, double* y, double alpha,
+                       double beta, int mode, cudaStream_t s);
+int launch_packed_spmv_dot(const Sell& A, const Packed64& P, const double* x, double* y, int n_dot,
+                           ReduceScratch rs, double* out, cudaStream_t s);
+
 // Generic launches used by several translation units.
 int launch_sell_spmv(const Sell& A, const double* vals, const double* x, double* y, double alpha,
                      double beta, int mode, cudaStream_t s);
@@ -236,6 +258,7 @@ int grid_blocks(int threads, int work_items, int per_thread, int max_blocks, int
 
 struct gipb200_matrix_s {
   gipb200::Sell S;
+  gipb200::Packed64 P;  // used while its values are S's (P.bits)
   // reduction scratch of the fused operations called on this handle (spmv_dot,
   // cg_update_dot): calls that share a handle must be ordered on one stream
   gipb200::DevBuf<double> partials;

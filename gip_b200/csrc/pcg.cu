@@ -1367,6 +1367,10 @@ static int host_poll_interval() {
 }
 
 int Pcg::enqueue(const double* b, double* x, const double* x0, cudaStream_t s, bool host_sync) {
+  if (op64.bits && L->version != packed_version) {  // L's values changed since they were packed
+    op64.bits = 0;
+    if (one.form == OneLaunch::kStream || one.form == OneLaunch::kSolve) one.form = OneLaunch::kNone;
+  }
   if (one_launch()) return enqueue_one_launch(b, x, x0, s);
   if (!host_sync && prm.mode != GIPB200_PCG_FIXED && capturing(s)) {
     if (!body_stream[0]) {

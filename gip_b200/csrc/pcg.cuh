@@ -56,18 +56,6 @@ struct CompressedOp {
   double bytes_per_launch = 0.0;     // stored bytes the kernel streams (+ vectors)
 };
 
-// The FP64 operator packed in GIP's slot order (build_packed64); bits = 0: not built.
-struct Packed64 {
-  int bits = 0;                  // value-table index bits: 4 or 8
-  int slots = 8;                 // 7: no packed row uses the eighth slot
-  DevBuf<uint4> delta;
-  DevBuf<unsigned> idx4;
-  DevBuf<uint2> idx8;
-  DevBuf<int> base;
-  DevBuf<unsigned char> plain;
-  DevBuf<double> table;
-};
-
 // How a whole solve runs as one launch; kNone: kernel by kernel.  kCluster, kGrid, kStream:
 // FP64 with GIP's Jacobi (persist.cu); kSolve: the mixed form and the FP64 tolerance mode
 // with AMG (persist_amg.cu).
@@ -150,7 +138,8 @@ struct Pcg {
   // constant mode is restored exactly from the pin equation.
   int pin_row = -1;
   double pin_val = 0.0;
-  Packed64 op64;
+  Packed64 op64;                 // L packed (bits = 0: not), at this version of its values
+  unsigned packed_version = 0;
   OneLaunch one;
   // several solvers advance side by side on one GPU (a batch): forms that claim every SM at
   // once (the cooperative ones) would take turns, so only the cluster form runs

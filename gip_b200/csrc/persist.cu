@@ -513,96 +513,9 @@ __global__ void __launch_bounds__(256, 8) k_pcg64_spmv_dot(SellView<double> L, S
 }  // namespace
 
 // ------------------------------------------------------------------ set-up
-// The packed layout of L in its stored slot order: eight 16-bit column deltas per row from a
-// base per (slice, slot) and eight indices into a table of L's values, as the mixed form
-// packs its FP32 operator (pcg.cu), but in GIP's order and in doubles.  Slots of ghost columns
-// (stored zeros) become padding.  Slices that do not fit keep the sliced layout.
 int Pcg::build_packed64(cudaStream_t s) {
-  const int ns = L->nslices;
-  const long long nslots = L->nslots;
-  if (ns == 0 || nslots == 0) return GIPB200_OK;
-  std::vector<long long> sptr((size_t)ns + 1);
-  std::vector<int> col((size_t)nslots);
-  std::vector<double> val((size_t)nslots);
-  GIPB_CUDA(cudaMemcpyAsync(sptr.data(), L->sptr.p, sptr.size() * 8, cudaMemcpyDeviceToHost, s));
-  GIPB_CUDA(cudaMemcpyAsync(col.data(), L->col.p, col.size() * 4, cudaMemcpyDeviceToHost, s));
-  GIPB_CUDA(cudaMemcpyAsync(val.data(), L->val.p, val.size() * 8, cudaMemcpyDeviceToHost, s));
-  GIPB_CUDA(cudaStreamSynchronize(s));
-  std::vector<double> tab;
-  if (!value_table(val.data(), nslots, 255, &tab)) return GIPB200_OK;
-  std::vector<unsigned long long> keys;
-  for (double t : tab)
-    if (t != 0.0 || std::signbit(t)) {
-      unsigned long long k;
-      memcpy(&k, &t, 8);
-      keys.push_back(k);
-    }
-  const int nib = keys.size() <= 15 ? 4 : 8;
-  std::vector<double> table((size_t)1 << nib, 0.0);
-  for (size_t t = 0; t < keys.size(); ++t) memcpy(&table[t + 1], &keys[t], 8);
-  const size_t rows = (size_t)ns * 32;
-  std::vector<uint4> delta(rows, make_uint4(0u, 0u, 0u, 0u));
-  std::vector<unsigned> idx4(nib == 4 ? rows : 0, 0u);
-  std::vector<uint2> idx8(nib == 8 ? rows : 0, make_uint2(0u, 0u));
-  std::vector<int> base((size_t)ns * 8, 0);
-  std::vector<unsigned char> plain((size_t)ns, 1);
-  long long packed = 0;
-  int longest = 0;
-  const int nu = n;
-#pragma omp parallel for schedule(static) reduction(+ : packed) reduction(max : longest)
-  for (int sl = 0; sl < ns; ++sl) {
-    const long long b0 = sptr[sl];
-    const int len = (int)((sptr[sl + 1] - b0) >> 5);
-    if (len > 8) continue;
-    int lo[8], hi[8];
-    bool ok = true;
-    for (int j = 0; j < len && ok; ++j) {
-      lo[j] = 0x7fffffff;
-      hi[j] = -1;
-      for (int l = 0; l < 32; ++l) {
-        const int c = col[b0 + 32LL * j + l];
-        if (c < 0 || c >= nu) continue;
-        lo[j] = std::min(lo[j], c);
-        hi[j] = std::max(hi[j], c);
-      }
-      ok = hi[j] < 0 || hi[j] - lo[j] <= 65535;
-    }
-    if (!ok) continue;
-    plain[sl] = 0;
-    packed += 1;
-    longest = std::max(longest, len);
-    for (int j = 0; j < len; ++j) base[(size_t)sl * 8 + j] = hi[j] >= 0 ? lo[j] : 0;
-    for (int l = 0; l < 32; ++l) {
-      unsigned dw[4] = {0u, 0u, 0u, 0u};
-      unsigned long long iw = 0ull;
-      for (int j = 0; j < len; ++j) {
-        const long long k = b0 + 32LL * j + l;
-        if (col[k] < 0 || col[k] >= nu) continue;
-        dw[j >> 1] |= (unsigned)(col[k] - lo[j]) << (16 * (j & 1));
-        unsigned long long bits;
-        memcpy(&bits, &val[k], 8);
-        if (bits == 0ull) continue;  // a stored +0.0: table entry 0
-        const unsigned t =
-            1u + (unsigned)(std::lower_bound(keys.begin(), keys.end(), bits) - keys.begin());
-        iw |= (unsigned long long)t << (nib * j);
-      }
-      const size_t r = (size_t)sl * 32 + l;
-      delta[r] = make_uint4(dw[0], dw[1], dw[2], dw[3]);
-      if (nib == 4) idx4[r] = (unsigned)iw;
-      else idx8[r] = make_uint2((unsigned)iw, (unsigned)(iw >> 32));
-    }
-  }
-  if (packed * 2 < ns) return GIPB200_OK;  // not worth a second layout
-  GIPB_TRY(op64.delta.upload(delta.data(), delta.size(), s));
-  if (nib == 4) GIPB_TRY(op64.idx4.upload(idx4.data(), idx4.size(), s));
-  else GIPB_TRY(op64.idx8.upload(idx8.data(), idx8.size(), s));
-  GIPB_TRY(op64.base.upload(base.data(), base.size(), s));
-  GIPB_TRY(op64.plain.upload(plain.data(), plain.size(), s));
-  GIPB_TRY(op64.table.upload(table.data(), table.size(), s));
-  GIPB_CUDA(cudaStreamSynchronize(s));
-  op64.bits = nib;
-  op64.slots = longest <= 7 ? 7 : 8;
-  return GIPB200_OK;
+  packed_version = L->version;
+  return pack64(*L, n, false, &op64, s);
 }
 
 namespace {
