@@ -194,8 +194,21 @@ def check(status: int, where: str) -> None:
         raise GipB200Error(status, where, lib.gipb200_last_error().decode(errors="replace"))
 
 
+_functions: dict = {}
+
+
+def function(name: str):
+    """The library's entry point `name` (looked up once)."""
+    fn = _functions.get(name)
+    if fn is None:
+        fn = _functions[name] = getattr(load(), name)
+    return fn
+
+
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args), name)
+    status = function(name)(*args)
+    if status != STATUS_OK:
+        check(status, name)
 
 
 def declared_symbols(header: str = None) -> list:

@@ -33,6 +33,7 @@ struct StoreDot {
 __global__ void __launch_bounds__(256, 8) k_spmv_dot(SellView<double> A, const double* __restrict__ x,
                                                      double* __restrict__ y, int n_dot,
                                                      ReduceScratch rs, double* out) {
+  dep_begin();
   const int lane = threadIdx.x & 31;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(256) k_cg_update(int n, double* __restrict__ x
                                                    const double* __restrict__ q,
                                                    const double* __restrict__ dinv,
                                                    gipb200_cg_scalars* sc, ReduceScratch rs) {
+  dep_begin();
   const double alpha = ddiv(sc->rz, sc->pAp);  // alpha = r1 / dn
   const double malpha = dmul(-1.0, alpha);
   double acc[2] = {0.0, 0.0};
@@ -116,6 +118,7 @@ template <bool V2>
 __global__ void __launch_bounds__(256) k_cg_direction(int n, double* __restrict__ p,
                                                       const double* __restrict__ z,
                                                       const gipb200_cg_scalars* sc) {
+  dep_begin();
   const double beta = sc->beta;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   int i0 = 0;
@@ -153,7 +156,7 @@ int gipb200_matrix_spmv_dot(gipb200_matrix A, const double* d_x, double* d_y, in
     return launch_packed_spmv_dot(A->S, A->P, d_x, d_y, n_dot, A->rs, d_dot, s);
   int blocks = 1;
   GIPB_TRY(grid_blocks(256, std::max(A->S.nslices, 1) * 32, 1, kMaxReduceBlocks, &blocks));
-  k_spmv_dot<<<blocks, 256, 0, s>>>(A->S.view(), d_x, d_y, n_dot, A->rs, d_dot);
+  launch_dep(k_spmv_dot, blocks, 256, s, A->S.view(), d_x, d_y, n_dot, A->rs, d_dot);
   GIPB_LAUNCH_CHECK();
   return GIPB200_OK;
 }
@@ -171,9 +174,9 @@ int gipb200_cg_update_dot(gipb200_matrix A, int n, double* d_x, double* d_r, dou
   const bool v2 = aligned16(d_x) && aligned16(d_r) && aligned16(d_z) && aligned16(d_p) &&
                   aligned16(d_q) && aligned16(d_dinv);
   if (v2)
-    k_cg_update<true><<<blocks, 256, 0, s>>>(n, d_x, d_r, d_z, d_p, d_q, d_dinv, d_sc, A->rs);
+    launch_dep(k_cg_update<true>, blocks, 256, s, n, d_x, d_r, d_z, d_p, d_q, d_dinv, d_sc, A->rs);
   else
-    k_cg_update<false><<<blocks, 256, 0, s>>>(n, d_x, d_r, d_z, d_p, d_q, d_dinv, d_sc, A->rs);
+    launch_dep(k_cg_update<false>, blocks, 256, s, n, d_x, d_r, d_z, d_p, d_q, d_dinv, d_sc, A->rs);
   GIPB_LAUNCH_CHECK();
   return GIPB200_OK;
 }
@@ -187,9 +190,9 @@ int gipb200_cg_direction(int n, double* d_p, const double* d_z, const gipb200_cg
   int blocks = 1;
   GIPB_TRY(grid_blocks(256, n, 4, 0, &blocks));
   if (aligned16(d_p) && aligned16(d_z))
-    k_cg_direction<true><<<blocks, 256, 0, s>>>(n, d_p, d_z, d_sc);
+    launch_dep(k_cg_direction<true>, blocks, 256, s, n, d_p, d_z, d_sc);
   else
-    k_cg_direction<false><<<blocks, 256, 0, s>>>(n, d_p, d_z, d_sc);
+    launch_dep(k_cg_direction<false>, blocks, 256, s, n, d_p, d_z, d_sc);
   GIPB_LAUNCH_CHECK();
   return GIPB200_OK;
 }

@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(256, 8) k_packed_spmv(SellView<double> A, Pack
                                                         double* __restrict__ y, double alpha,
                                                         double beta, int mode, int n_dot,
                                                         ReduceScratch rs, double* out) {
+  dep_begin();
   __shared__ double tab[NIB == 4 ? 16 : 256];
   for (int t = threadIdx.x; t < (NIB == 4 ? 16 : 256); t += blockDim.x) tab[t] = M.table[t];
   __syncthreads();
@@ -184,11 +185,11 @@ int launch(const Sell& A, const Packed64& P, const double* x, double* y, double 
   GIPB_TRY(P.bits == 4 ? one_wave(k_packed_spmv<4, DOT>, (A.nslices * 32 + 255) / 256, &blocks)
                        : one_wave(k_packed_spmv<8, DOT>, (A.nslices * 32 + 255) / 256, &blocks));
   if (P.bits == 4)
-    k_packed_spmv<4, DOT><<<blocks, 256, 0, s>>>(A.view(), args_of(P), x, y, alpha, beta, mode,
-                                                 n_dot, rs, out);
+    launch_dep(k_packed_spmv<4, DOT>, blocks, 256, s, A.view(), args_of(P), x, y, alpha, beta,
+               mode, n_dot, rs, out);
   else
-    k_packed_spmv<8, DOT><<<blocks, 256, 0, s>>>(A.view(), args_of(P), x, y, alpha, beta, mode,
-                                                 n_dot, rs, out);
+    launch_dep(k_packed_spmv<8, DOT>, blocks, 256, s, A.view(), args_of(P), x, y, alpha, beta,
+               mode, n_dot, rs, out);
   GIPB_LAUNCH_CHECK();
   return GIPB200_OK;
 }

@@ -18,8 +18,8 @@ from .formats import Csr, GipCase
 
 
 def _stream(stream=None) -> C.c_void_p:
-    if stream is None:
-        stream = torch.cuda.current_stream()
+    if stream is None:  # the current stream's handle, without building a Stream object
+        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
     return C.c_void_p(stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream))
 
 
@@ -285,11 +285,17 @@ def host_loop_pcg(A: DeviceMatrix, Dg: DeviceMatrix, dinv: torch.Tensor, b: torc
     A.spmv(x, Ax, stream=stream)       # dAx = A x
     L.call("gipb200_daxpy", n, _dptr(r), _dptr(Ax), -1.0, s)  # dr += -1 dAx
     Dg.spmv_dot(r, p, sc, n_dot=n, stream=stream)              # dp = D r; r1 = r.dp
+    # the iterations' arguments, converted once (the loop is bound by the host: three calls an
+    # iteration)
+    spmv_dot, update, direction = (L.function("gipb200_" + f) for f in
+                                   ("matrix_spmv_dot", "cg_update_dot", "cg_direction"))
     pAp = C.c_void_p(sc.data_ptr() + 8)
+    dp, dAx, dx, dr, dz, dd, dsc = (_dptr(t) for t in (p, Ax, x, r, z, dinv, sc))
     for _ in range(maxit):
-        L.call("gipb200_matrix_spmv_dot", A.handle, _dptr(p), _dptr(Ax), n, pAp, s)
-        cg_update_dot(A, n, x, r, z, p, Ax, dinv, sc, stream)
-        cg_direction(n, p, z, sc, stream)
+        st = spmv_dot(A.handle, dp, dAx, n, pAp, s) or \
+            update(A.handle, n, dx, dr, dz, dp, dAx, dd, dsc, s) or direction(n, dp, dz, dsc, s)
+        if st:
+            L.check(st, "host_loop_pcg")
     return sc
 
 
