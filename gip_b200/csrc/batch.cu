@@ -1,6 +1,9 @@
 // Batched cavities: one CUDA graph per timestep.  By default each instance's whole step is
 // a parallel branch (fork/join events) with its own conditional PCG loops (pcg.cu), so
-// instances converge independently inside the same launch.  With the persistent solver the
+// instances converge independently inside the same launch.  When every instance is mixed with
+// AMG and the systems are small (SolveGroups::plan has the rule and both sides' times), the
+// branches stop before the pressure solve and one cooperative launch solves all of them, a CTA
+// group per instance.  With the persistent solver (mixed with Jacobi, on request) the
 // branches stop before the pressure solve, one cooperative launch (batch_pcg.cu) solves
 // every instance's pressure system with a CTA group per instance, and a second set of
 // branches finishes the steps.
@@ -32,6 +35,9 @@ struct Batch {
   DevBuf<unsigned> d_bar;
   DevBuf<double> d_part;
   DevBuf<int> d_err;
+  // mixed AMG solves of all instances in one launch (not with the persistent Jacobi solve)
+  SolveGroups groups;
+  int plan_groups();
   ~Batch() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -65,21 +71,45 @@ int Batch::branches(cudaEvent_t from, int part, int* st) {
     E.graph_kernels += E.launches - before;
     E.launches = before;
     if (*st != GIPB200_OK) return *st;
+    if (part == 1 && !persistent && E.pcg.lpacked) {  // what the grouped solve starts from
+      const double* bp = nullptr;
+      *st = E.pcg.enqueue_ghost_rhs(E.rhs.p, E.p0.p, streams[i], &bp);
+      if (*st != GIPB200_OK) return *st;
+    }
     GIPB_CUDA(cudaEventRecord(joins[i], streams[i]));
     GIPB_CUDA(cudaStreamWaitEvent(cap, joins[i], 0));
   }
   return GIPB200_OK;
 }
 
+int Batch::plan_groups() {
+  std::vector<Pcg*> solvers;
+  std::vector<const double*> b, x0;
+  std::vector<double*> x;
+  for (auto d : inst) {
+    solvers.push_back(&d->E.pcg);
+    b.push_back(d->E.rhs.p);
+    x.push_back(d->E.p.p);
+    x0.push_back(d->E.p0.p);
+  }
+  return groups.plan(solvers, b, x, x0, cap);
+}
+
 int Batch::capture() {
   for (auto d : inst) d->E.graph_kernels = 0;
+  groups.on = false;
+  if (!persistent) GIPB_TRY(plan_groups());
   GIPB_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
   int st = GIPB200_OK;
   int rc = [&]() -> int {
-    if (!persistent) return branches(fork, 0, &st);
+    if (!persistent && !groups.on) return branches(fork, 0, &st);
     GIPB_TRY(branches(fork, 1, &st));
-    GIPB_CUDA(cudaMemsetAsync(d_bar.p, 0, inst.size() * sizeof(unsigned), cap));
-    GIPB_TRY(batch_pcg_launch(shape, grid, d_inst.p, d_owner.p, d_err.p, cap));
+    if (groups.on) {
+      GIPB_TRY(groups.launch(cap));
+    } else {
+      GIPB_CUDA(cudaMemsetAsync(d_bar.p, 0, inst.size() * sizeof(unsigned), cap));
+      GIPB_TRY(batch_pcg_launch(shape, grid, d_inst.p, d_owner.p, d_err.p, cap));
+    }
     inst[0]->E.graph_kernels += 1;
     return branches(fork2, 2, &st);
   }();

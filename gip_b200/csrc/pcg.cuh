@@ -183,14 +183,15 @@ struct Pcg {
   std::vector<int> cycle_forms;  // kernel forms of the last profiled cycle (GIPB200_FORM_*)
   int vcycle_forms(int cap, int* n_kernels, int* h_form) const;
 
+  // b less L's ghost part into bprime (*bp: bprime, or b itself without ghost rows)
+  int enqueue_ghost_rhs(const double* b, const double* x, cudaStream_t s, const double** bp);
+
  private:
   int build_packed64(cudaStream_t s);
   int plan_one_launch(cudaStream_t s);
   int plan_solve_launch(cudaStream_t s);
   int enqueue_solve_launch(const double* b, double* x, const double* x0, cudaStream_t s);
   int ghosts_zero(cudaStream_t s, bool* zero) const;  // L's ghost columns all hold 0.0
-  // b less L's ghost part into bprime (*bp: bprime, or b itself without ghost rows)
-  int enqueue_ghost_rhs(const double* b, const double* x, cudaStream_t s, const double** bp);
   void launch_packed64_spmv(double* q, PcgScalars* S, int mode, cudaStream_t s);
   // operator bytes a product streams from the packed FP64 layout: column deltas, value
   // indices, the slices' slot bases
@@ -205,6 +206,19 @@ struct Pcg {
   int launch_mixed_residual(const double* b, const double* bp, const double* x, int first,
                             cudaStream_t s,
                             int use_cond, cudaGraphConditionalHandle h);
+};
+
+// The mixed AMG solves of several solvers (a batch's) in one cooperative launch, a group of
+// CTAs each; on = false: some solver's solve does not run as one launch.
+struct SolveGroups {
+  bool on = false;
+  int ctas = 0;
+  DevBuf<unsigned char> items;   // the solves' arguments
+  DevBuf<int> owner;             // solver of every CTA
+  DevBuf<ulonglong2> slots;      // the groups' barriers
+  int plan(const std::vector<Pcg*>& solvers, const std::vector<const double*>& b,
+           const std::vector<double*>& x, const std::vector<const double*>& x0, cudaStream_t s);
+  int launch(cudaStream_t s) const;
 };
 
 }  // namespace gipb200

@@ -191,6 +191,7 @@ struct SolveArgs {
   double tol, delta, pin_val;
   int n, n_all, maxit, max_outer, pin_row;
   int nib;                  // value-table index bits of the packed operator, 0: not packed
+  int count;                // launches the solve's scalars report
 };
 
 struct State {
@@ -932,7 +933,7 @@ __device__ __forceinline__ void mixed_solve(const SolveArgs<float>& A, Team& g) 
     S->status = ok ? T.status : GIPB200_ERR_TIMEOUT;
     S->outer = T.outer;
     S->total_inner = T.total;
-    S->kernels = 1;
+    S->kernels = A.count;
     S->kappa_c = T.kappa_c;
     S->kappa = T.kappa;
     S->maxr2 = T.maxr2;
@@ -959,6 +960,25 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed_cluster(const __grid_cons
   ClusterTeam g = cluster_team(red);
   mixed_solve<AMG>(A, g);
   cluster_barrier();  // no CTA leaves while another may still write its sums
+}
+
+// The solves of a batch in one launch, a group of CTAs per instance; groups never wait on one
+// another and leave when their instance has converged.
+struct GroupSolve {
+  SolveArgs<float> A;
+  int cta0, ncta;
+};
+__global__ void __launch_bounds__(kThreads, 1) k_mixed_groups(const GroupSolve* __restrict__ all,
+                                                              const int* __restrict__ owner) {
+  __shared__ GroupSolve I;
+  const int who = owner[blockIdx.x];
+  if (who < 0) return;  // the groups do not fill the grid
+  static_assert(sizeof(GroupSolve) % 4 == 0, "copied in words");
+  for (int k = threadIdx.x; k < (int)(sizeof(GroupSolve) / 4); k += kThreads)
+    reinterpret_cast<unsigned*>(&I)[k] = reinterpret_cast<const unsigned*>(all + who)[k];
+  __syncthreads();
+  GridTeam g{grid_begin(I.A.slots, (int)blockIdx.x - I.cta0, I.ncta)};
+  mixed_solve<true>(I.A, g);
 }
 
 // ------------------------------------------------------------------ FP64 tolerance mode, AMG
@@ -1305,45 +1325,53 @@ int Pcg::plan_solve_launch(cudaStream_t s) {
   return one.slots.alloc(grid_slot_count(one.ctas));
 }
 
+namespace {
+SolveArgs<float> mixed_args(Pcg& P, const double* b, const double* bp, double* x, const double* x0) {
+  SolveArgs<float> A{};
+  const PackedView pk = P.packed();
+  A.op = {P.a32(), pk.delta, pk.idx, pk.base, pk.plain, pk.table, pk.slots, P.n};
+  A.L = P.L->view();
+  A.lidx = P.lpacked ? P.lidx4.p : nullptr;
+  A.ltable = P.ltable.p;
+  A.bp = bp;
+  A.b = b;
+  A.x0 = x0;
+  A.x = x;
+  A.scale = P.scale.p;
+  A.pair = reinterpret_cast<float2*>(P.one.pair.p);
+  A.r = P.r32.p;
+  A.q = P.Ap32.p;
+  A.y = P.y32.p;
+  A.rd = P.one.rd.p;
+  A.rpart = P.one.rd.p + P.n;
+  A.vblocks = P.blocks_spmv;
+  A.S = P.sc.p;
+  A.slots = P.one.slots.p;
+  A.ops = reinterpret_cast<const CycleOp<float>*>(P.one.ops.p);
+  A.nops = P.one.nops;
+  if (P.amg) cycle_args<float>(*P.amg, &A);
+  A.tol = P.prm.tol;
+  A.delta = P.prm.inner_tol;
+  A.pin_val = P.pin_val;
+  A.n = P.n;
+  A.n_all = P.n_all;
+  A.maxit = P.prm.maxit;
+  A.max_outer = P.prm.max_outer;
+  A.pin_row = P.pin_row;
+  A.nib = pk.on ? pk.nib : 0;
+  A.count = 1;
+  return A;
+}
+}  // namespace
+
 int Pcg::enqueue_solve_launch(const double* b, double* x, const double* x0, cudaStream_t s) {
   if (!one.cluster)
     GIPB_CUDA(cudaMemsetAsync(one.slots.p, 0, one.slots.n * sizeof(ulonglong2), s));
   launches += 1;
   if (prm.mode == GIPB200_PCG_MIXED) {
-    SolveArgs<float> A{};
     const double* bp = b;
     if (lpacked) GIPB_TRY(enqueue_ghost_rhs(b, x0, s, &bp));
-    const PackedView pk = packed();
-    A.op = {a32(), pk.delta, pk.idx, pk.base, pk.plain, pk.table, pk.slots, n};
-    A.L = L->view();
-    A.lidx = lpacked ? lidx4.p : nullptr;
-    A.ltable = ltable.p;
-    A.bp = bp;
-    A.b = b;
-    A.x0 = x0;
-    A.x = x;
-    A.scale = scale.p;
-    A.pair = reinterpret_cast<float2*>(one.pair.p);
-    A.r = r32.p;
-    A.q = Ap32.p;
-    A.y = y32.p;
-    A.rd = one.rd.p;
-    A.rpart = one.rd.p + n;
-    A.vblocks = blocks_spmv;
-    A.S = sc.p;
-    A.slots = one.slots.p;
-    A.ops = reinterpret_cast<const CycleOp<float>*>(one.ops.p);
-    A.nops = one.nops;
-    if (amg) cycle_args<float>(*amg, &A);
-    A.tol = prm.tol;
-    A.delta = prm.inner_tol;
-    A.pin_val = pin_val;
-    A.n = n;
-    A.n_all = n_all;
-    A.maxit = prm.maxit;
-    A.max_outer = prm.max_outer;
-    A.pin_row = pin_row;
-    A.nib = pk.on ? pk.nib : 0;
+    const SolveArgs<float> A = mixed_args(*this, b, bp, x, x0);
     if (one.cluster)
       return amg ? launch_solve(k_mixed_cluster<true>, one, A, s)
                  : launch_solve(k_mixed_cluster<false>, one, A, s);
@@ -1374,6 +1402,83 @@ int Pcg::enqueue_solve_launch(const double* b, double* x, const double* x0, cuda
   A.nib = o.bits;
   return one.cluster ? launch_solve(k_tol_amg_cluster, one, A, s)
                      : launch_solve(k_tol_amg_grid, one, A, s);
+}
+
+// ------------------------------------------------------------------ groups
+int SolveGroups::plan(const std::vector<Pcg*>& solvers, const std::vector<const double*>& b,
+                      const std::vector<double*>& x, const std::vector<const double*>& x0,
+                      cudaStream_t s) {
+  on = false;
+  const int ni = (int)solvers.size();
+  DeviceInfo di;
+  GIPB_TRY(device_info(&di));
+  ctas = std::min(di.nsm, kGridCtasMax);
+  if (ni > ctas) return GIPB200_OK;
+  double rows = 0.0;
+  for (const Pcg* P : solvers) {
+    if (P->prm.mode != GIPB200_PCG_MIXED || !P->amg || P->one.form != OneLaunch::kSolve)
+      return GIPB200_OK;
+    rows += P->n;
+  }
+  // Batches of small systems, or a small batch: the branches' kernels reach a higher rate once
+  // they fill the chip.  Measured per step, branches / groups: 3 of 12..20 edges 0.63 / 0.46
+  // ms, 8 of 20..30 1.4 / 1.0, 32 of 16..48 (37k rows on average) 6.0 / 4.2, 2 of 44 1.08 /
+  // 0.82; 12 of 24..64 (103k) 3.8 / 3.7, 16 of 32..64 (120k) 4.5 / 5.2, 6 of 64..77 4.1 / 6.0.
+  if (rows > 600000.0 && rows > 60000.0 * ni) return GIPB200_OK;
+  // CTAs by rows (the instances' iteration counts are close with AMG): at least one each
+  std::vector<int> share(ni);
+  int used = 0;
+  for (int i = 0; i < ni; ++i) {
+    share[i] = std::max(1, (int)((double)ctas * solvers[i]->n / rows));
+    used += share[i];
+  }
+  for (; used > ctas; --used) *std::max_element(share.begin(), share.end()) -= 1;
+  for (; used < ctas; ++used) {  // the rest to the instances with the most rows per CTA
+    int k = 0;
+    for (int i = 1; i < ni; ++i)
+      if ((double)solvers[i]->n * share[k] > (double)solvers[k]->n * share[i]) k = i;
+    share[k] += 1;
+  }
+  size_t need = 0;
+  for (int i = 0; i < ni; ++i) need += grid_slot_count(share[i]);
+  GIPB_TRY(slots.alloc(need));
+  std::vector<GroupSolve> h(ni);
+  std::vector<int> own(ctas, -1);
+  size_t at = 0;
+  int c = 0;
+  for (int i = 0; i < ni; ++i) {
+    Pcg& P = *solvers[i];
+    const bool ghosts = P.lpacked && !P.ghost_rows.empty();
+    h[i].A = mixed_args(P, b[i], ghosts ? P.bprime.p : b[i], x[i], x0[i]);
+    h[i].A.slots = slots.p + at;
+    h[i].A.count = i == 0 ? 1 : 0;
+    h[i].cta0 = c;
+    h[i].ncta = share[i];
+    for (int k = 0; k < share[i]; ++k) own[c + k] = i;
+    c += share[i];
+    at += grid_slot_count(share[i]);
+  }
+  GIPB_TRY(items.upload(reinterpret_cast<const unsigned char*>(h.data()), ni * sizeof(GroupSolve), s));
+  GIPB_TRY(owner.upload(own.data(), own.size(), s));
+  GIPB_CUDA(cudaStreamSynchronize(s));
+  on = true;
+  return GIPB200_OK;
+}
+
+int SolveGroups::launch(cudaStream_t s) const {
+  GIPB_CUDA(cudaMemsetAsync(slots.p, 0, slots.n * sizeof(ulonglong2), s));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  GIPB_CUDA(cudaLaunchKernelEx(&cfg, k_mixed_groups, reinterpret_cast<const GroupSolve*>(items.p),
+                               (const int*)owner.p));
+  return GIPB200_OK;
 }
 
 }  // namespace gipb200

@@ -222,3 +222,33 @@ def test_preconditioned_one_launch_layouts(gpu, monkeypatch, values, far):
         rs, rk = S.solve(_t(b), xs, _t(np.zeros(n))), K.solve(_t(b), xk, _t(np.zeros(n)))
         assert rs["status"] == rk["status"] == 0, (solve, rs, rk)
         assert float((xs - xk).abs().max()) <= 1e-8 * float(xk.abs().max()), solve
+
+
+@pytest.mark.parametrize("edges", [[12, 17, 16, 24, 9], [10, 10], [40, 8, 20]])
+def test_grouped_batch_solves_equal_the_branches(gpu, monkeypatch, edges):
+    # a batch's mixed AMG solves in one launch, a CTA group per instance, against the same
+    # batch solving inside its graph branches and against single engines: the same steps
+    from gip_b200 import cavity
+    from gip_b200.device import DnsBatch, DnsEngine, dns_params
+    cases = [cavity.generate(n, re=100.0 * (i + 1), permute_seed=i)[0] for i, n in enumerate(edges)]
+    kw = dict(pcg_mode="mixed", maxit=2000, tol=1e-8, inner_tol=1e-2, max_outer=100, reorder=True,
+              precond="amg")
+    prm = [dns_params(gamma=1.0 / (100.0 * (i + 1)), **kw) for i in range(len(edges))]
+    G = DnsBatch(cases, prm)
+    single = DnsEngine(cases[0], gamma=1.0 / 100.0, **kw)
+    monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+    B = DnsBatch(cases, prm)
+    for batch in (G, B, single):
+        batch.advance(2)
+        batch.advance(1)
+    assert np.all(G.instances[0].history()["kernels"] == 11)   # one launch, counted once
+    assert all(np.all(e.history()["kernels"] == 10) for e in G.instances[1:])
+    assert np.all(B.instances[0].history()["kernels"] > 11)
+    for e, f in zip(G.instances, B.instances):
+        he, hf = e.history(), f.history()
+        assert np.all(he["massr"] < 1e-6) and np.all(np.abs(he["iters"] - hf["iters"]) <= 1)
+        scale = np.abs(f.field("u")).max()
+        for k in ("u", "v", "w"):
+            assert np.abs(e.field(k) - f.field(k)).max() <= 1e-9 * scale, k
+    for k in ("u", "v", "w"):
+        assert np.abs(G.instances[0].field(k) - single.field(k)).max() <= 1e-9 * np.abs(single.field("u")).max()
