@@ -387,12 +387,12 @@ __device__ __forceinline__ void row_store(const CycleOp<T>& o, int i, const RowO
 // running sum passes from thread to thread, so a row is still one chain of FMAs in slot
 // order, but a row of 29 slots costs one round trip instead of four.
 template <typename T, int LANES>
-__device__ __forceinline__ void sell_unit(const CycleOp<T>& o, Ahead<T>& a) {
+__device__ __forceinline__ void sell_unit(const CycleOp<T>& o, int u, int& k, int& len) {
   constexpr int RPW = 32 / LANES;
-  const int lane = threadIdx.x & 31, s = a.u / LANES;
+  const int lane = threadIdx.x & 31, s = u / LANES;
   const int b0 = (int)__ldg(o.sptr + s);
-  a.len = ((int)__ldg(o.sptr + s + 1) - b0) >> 5;
-  a.k = b0 + (a.u % LANES) * RPW + lane / LANES;
+  len = ((int)__ldg(o.sptr + s + 1) - b0) >> 5;
+  k = b0 + (u % LANES) * RPW + lane / LANES;
 }
 template <typename T, typename V, bool XS, int LANES>
 __device__ __forceinline__ void sell_run(const CycleOp<T>& o, Ahead<T>& a) {
@@ -402,6 +402,8 @@ __device__ __forceinline__ void sell_run(const CycleOp<T>& o, Ahead<T>& a) {
     const int i = (a.u / LANES) * 32 + (a.u % LANES) * RPW + lane / LANES;
     const bool writes = i < o.nrows && sub == 0;
     const RowOps<T> r = row_ops(o, i, writes);
+    int k1 = 0, len1 = 0;  // the warp's next unit
+    if (a.u + nw < a.uend) sell_unit<T, LANES>(o, a.u + nw, k1, len1);
     T sum = T(0);
     for (int j0 = 0;;) {
       T xv[8], v[8];
@@ -412,9 +414,10 @@ __device__ __forceinline__ void sell_run(const CycleOp<T>& o, Ahead<T>& a) {
       const bool last = j0 >= a.len;
       if (last) {
         a.u += nw;
-        if (a.u < a.uend) sell_unit<T, LANES>(o, a);
+        a.k = k1;
+        a.len = len1;
       }
-      if (!last || a.u < a.uend) load8<T, V, 1, 32>(o, a.k, (last ? 0 : j0) + 8 * sub, a.len, a);
+      load8<T, V, 1, 32>(o, a.k, (last ? 0 : j0) + 8 * sub, a.len, a);
 #pragma unroll
       for (int q = 0; q < LANES; ++q) {
         T part = sum;
@@ -428,14 +431,15 @@ __device__ __forceinline__ void sell_run(const CycleOp<T>& o, Ahead<T>& a) {
   }
 }
 
-// CSR rows, LANES threads per row, each adding a strided part, combined by a fixed tree
+// CSR rows, LANES threads per row, each adding a strided part, combined by a fixed tree,
+// the next unit's loads as above
 template <typename T, int LANES>
-__device__ __forceinline__ void csr_unit(const CycleOp<T>& o, Ahead<T>& a) {
-  const int i = a.u * (32 / LANES) + (int)(threadIdx.x & 31) / LANES;
-  a.k = a.len = 0;
+__device__ __forceinline__ void csr_unit(const CycleOp<T>& o, int u, int& k, int& len) {
+  const int i = u * (32 / LANES) + (int)(threadIdx.x & 31) / LANES;
+  k = len = 0;
   if (i < o.nrows) {
-    a.k = __ldg(o.rp + i);
-    a.len = __ldg(o.rp + i + 1) - a.k;
+    k = __ldg(o.rp + i);
+    len = __ldg(o.rp + i + 1) - k;
   }
 }
 template <typename T, typename V, bool XS, int LANES>
@@ -445,26 +449,35 @@ __device__ __forceinline__ void csr_run(const CycleOp<T>& o, Ahead<T>& a) {
     const int i = a.u * (32 / LANES) + lane / LANES;
     const bool writes = i < o.nrows && sub == 0;
     const RowOps<T> r = row_ops(o, i, writes);
+    int k1 = 0, len1 = 0;
+    if (a.u + nw < a.uend) csr_unit<T, LANES>(o, a.u + nw, k1, len1);
     T sum = T(0);
     for (int q0 = sub;;) {
-      T xv[8];
+      T xv[8], v[8];
       gather8<T, XS>(o, a, xv);
+      unsigned in = 0;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        v[t] = a.v[t];
+        in |= (a.c[t] >= 0 ? 1u : 0u) << t;
+      }
+      q0 += 8 * LANES;
+      const bool more = __any_sync(0xffffffffu, q0 < a.len);
+      if (!more) {
+        a.k = k1;
+        a.len = len1;
+        q0 = sub;
+      }
+      load8<T, V, LANES, 1>(o, a.k, q0, a.len, a);
 #pragma unroll
       for (int t = 0; t < 8; ++t)
-        if (a.c[t] >= 0) sum = fmat(a.v[t], xv[t], sum);
-      q0 += 8 * LANES;
-      if (q0 >= a.len) break;
-      load8<T, V, LANES, 1>(o, a.k, q0, a.len, a);
+        if (in >> t & 1u) sum = fmat(v[t], xv[t], sum);
+      if (!more) break;
     }
-    __syncwarp();
 #pragma unroll
     for (int d = LANES / 2; d > 0; d >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, d, LANES);
     if (writes) row_store(o, i, r, sum);
     a.u += nw;
-    if (a.u < a.uend) {
-      csr_unit<T, LANES>(o, a);
-      load8<T, V, LANES, 1>(o, a.k, sub, a.len, a);
-    }
   }
 }
 
@@ -506,26 +519,26 @@ __device__ __forceinline__ void first_load(const CycleOp<T>& o, Ahead<T>& a) {
   const int lane = threadIdx.x & 31;
   if (o.form == kSell) {
     if (o.lanes == 4) {
-      sell_unit<T, 4>(o, a);
+      sell_unit<T, 4>(o, a.u, a.k, a.len);
       load8<T, V, 1, 32>(o, a.k, 8 * (lane % 4), a.len, a);
     } else if (o.lanes == 2) {
-      sell_unit<T, 2>(o, a);
+      sell_unit<T, 2>(o, a.u, a.k, a.len);
       load8<T, V, 1, 32>(o, a.k, 8 * (lane % 2), a.len, a);
     } else {
-      sell_unit<T, 1>(o, a);
+      sell_unit<T, 1>(o, a.u, a.k, a.len);
       load8<T, V, 1, 32>(o, a.k, 0, a.len, a);
     }
   } else if (o.lanes == 32) {
-    csr_unit<T, 32>(o, a);
+    csr_unit<T, 32>(o, a.u, a.k, a.len);
     load8<T, V, 32, 1>(o, a.k, lane, a.len, a);
   } else if (o.lanes == 16) {
-    csr_unit<T, 16>(o, a);
+    csr_unit<T, 16>(o, a.u, a.k, a.len);
     load8<T, V, 16, 1>(o, a.k, lane % 16, a.len, a);
   } else if (o.lanes == 8) {
-    csr_unit<T, 8>(o, a);
+    csr_unit<T, 8>(o, a.u, a.k, a.len);
     load8<T, V, 8, 1>(o, a.k, lane % 8, a.len, a);
   } else {
-    csr_unit<T, 4>(o, a);
+    csr_unit<T, 4>(o, a.u, a.k, a.len);
     load8<T, V, 4, 1>(o, a.k, lane % 4, a.len, a);
   }
 }
