@@ -1339,6 +1339,7 @@ int AmgT<T>::build(int n, const int* rp, const int* ci, const double* v, const d
   }));
   op_complexity = nnz_all / std::max(nnz0, 1.0);
   GIPB_TRY(build_tail(s));
+  GIPB_TRY(plan_small_levels(*this, s));
   GIPB_CUDA(cudaStreamSynchronize(s));
   setup_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   return GIPB200_OK;
@@ -1488,7 +1489,9 @@ int AmgT<T>::enqueue(SellView<T> A0, const T* r, T* z0, PcgScalars* S, ReduceScr
   auto a_bytes = [&](int l) { return l == 0 ? a0_stream_bytes : stream_bytes(lv[l]->A); };
   // downward: pre-smooth from zero, residual, restriction (levels below the coarse tail)
   const bool u0 = unit0;  // level 0 never forms x0 = omega0 r
-  const int tf = tail_from;
+  // a traced cycle runs kernel by kernel: its products are timed one by one
+  const bool small = tail_from < 0 && small_from > 0 && !tr;
+  const int tf = small ? small_from : tail_from;
   for (int l = 0; l < L - 1 && (tf < 0 || l < tf); ++l) {
     const AmgLevel<T>& V = *lv[l];
     const T* b = l == 0 ? r : V.b.p;
@@ -1523,7 +1526,9 @@ int AmgT<T>::enqueue(SellView<T> A0, const T* r, T* z0, PcgScalars* S, ReduceScr
     amg_mv<T, kPlain>(V.R, V.t.p, (const T*)nullptr, (const T*)nullptr, lv[l + 1]->b.p, S, s);
   }
   const AmgLevel<T>& C = *lv[L - 1];
-  if (tf >= 0) {  // the small levels and the coarsest in one cooperative launch
+  if (small) {  // the small levels and the coarsest, one launch of one cluster
+    GIPB_TRY(launch_small_levels(*this, S, s));
+  } else if (tf >= 0) {  // the small levels and the coarsest in one cooperative launch
     GIPB_TRY(mark(tf, GIPB200_CYCLE_TAIL, tail_bytes, GIPB200_FORM_TAIL));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)tail_grid);

@@ -136,6 +136,10 @@ struct AmgT {
   double tail_bytes = 0.0;
   int build_tail(cudaStream_t s);
   int reset_tail(cudaStream_t s) const;
+  // Small levels (small_from.. and the dense coarsest solve) in one launch of one cluster
+  // (persist_amg.cu); small_from < 0: one kernel per product.
+  int small_from = -1, small_nops = 0, small_ctas = 0;
+  DevBuf<unsigned char> small_ops;
 
   // Hierarchy of the n x n operator (host CSR, FP64 values; columns < n), near-null
   // vector z.  singular: the operator annihilates z (pinned-Neumann inner system), so the
@@ -173,6 +177,12 @@ double stream_bytes(const SellT<T>& M) {
   return (double)M.nslots * ((M.short_cols ? 2.0 : 4.0) + w) + (M.nslices + 1.0) * 8.0 +
          (M.short_cols ? 4.0 * M.nrows : 0.0);
 }
+
+// The small levels' launch: which levels, and the launch itself.
+template <typename T>
+int plan_small_levels(AmgT<T>& M, cudaStream_t s);
+template <typename T>
+int launch_small_levels(const AmgT<T>& M, PcgScalars* S, cudaStream_t s);
 
 using Amg = AmgT<float>;
 using Amg64 = AmgT<double>;

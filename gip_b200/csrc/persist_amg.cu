@@ -1158,6 +1158,33 @@ __global__ void __launch_bounds__(kThreads, 1) k_tol_amg_cluster(const __grid_co
   cluster_barrier();
 }
 
+// ------------------------------------------------------------------ small levels
+// The V-cycle's small levels and the dense coarsest solve in one launch of one cluster, for
+// cycles whose other levels run kernel by kernel.  Every product costs latency only: in a
+// captured step about 3 us as a kernel of its own, 2 to 3 us here, a cluster barrier after the
+// last; the launches they no longer need are what a batch's branches compete for.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 1) k_amg_small(const CycleOp<T>* __restrict__ all, int nops,
+                                                           PcgScalars* S) {
+  __shared__ CycleOp<T> ops[kMaxOps];
+  for (int k = threadIdx.x; k < (int)(nops * sizeof(CycleOp<T>) / 4); k += kThreads)
+    reinterpret_cast<unsigned*>(ops)[k] = reinterpret_cast<const unsigned*>(all)[k];
+  __syncthreads();
+  ClusterTeam g{nullptr, (int)blockIdx.x, (int)gridDim.x, 0};
+  Ahead<T> w;
+  product_ahead<T>(ops[0], g, w);
+  dep_begin();
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&S->kernels, 1);
+  if (S->done != 0) return;
+  product_run<T>(ops[0], w);
+  for (int k = 1; k < nops; ++k) {
+    g.arrive();
+    product_ahead<T>(ops[k], g, w);
+    g.wait();
+    product_run<T>(ops[k], w);
+  }
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ set-up
@@ -1416,6 +1443,60 @@ int Pcg::enqueue_solve_launch(const double* b, double* x, const double* x0, cuda
   return one.cluster ? launch_solve(k_tol_amg_cluster, one, A, s)
                      : launch_solve(k_tol_amg_grid, one, A, s);
 }
+
+// ------------------------------------------------------------------ small levels
+template <typename T>
+int plan_small_levels(AmgT<T>& M, cudaStream_t s) {
+  M.small_from = -1;
+  const int L = (int)M.lv.size();
+  if (L < 3 || M.nc <= 0 || getenv("GIPB200_NO_ONE_LAUNCH")) return GIPB200_OK;
+  // Levels whose operator streams at most 1 MB: 16 SMs read a larger one slower than the whole
+  // GPU.  Restart, steps and reads in ms by largest operator, none / 0.3 / 1 / 2 / 4 / 16 MB: 12
+  // cavities of 24..64 edges 10.3 / 10.0 / 10.0 / 10.1 / 10.2 / 10.5, 100^3 19.7 / 19.6 / 18.9 /
+  // 18.8 / 18.6 / 18.8, 160^3 28.0 / 28.0 / 28.0 / 28.0 / 28.8 / 28.7; a cluster of 8 is slower
+  // (19.3 at 100^3).
+  constexpr double most = 1e6;
+  int t = L - 1;
+  while (t - 1 >= 1 && stream_bytes(M.lv[t - 1]->A) <= most) --t;
+  if (t > L - 2) return GIPB200_OK;
+  OneLaunch o;
+  o.cluster = true;
+  o.ctas = ClusterTeam::kMaxCtas;
+  if (!cluster_fits(k_amg_small<T>, o)) return GIPB200_OK;
+  std::vector<CycleOp<T>> ops;
+  if (!cycle_ops<T>(M, (const T*)nullptr, o.ctas * (kThreads / 32), &ops)) return GIPB200_OK;
+  const int first = 2 * t - 1, count = (int)ops.size() - 2 * first;
+  GIPB_TRY(M.small_ops.upload(reinterpret_cast<const unsigned char*>(ops.data() + first),
+                              count * sizeof(CycleOp<T>), s));
+  GIPB_CUDA(cudaStreamSynchronize(s));
+  M.small_nops = count;
+  M.small_ctas = o.ctas;
+  M.small_from = t;
+  return GIPB200_OK;
+}
+
+template <typename T>
+int launch_small_levels(const AmgT<T>& M, PcgScalars* S, cudaStream_t s) {
+  OneLaunch o;
+  o.cluster = true;
+  o.ctas = M.small_ctas;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at[2];
+  solve_config(k_amg_small<T>, o, &cfg, at);
+  if (dependent_launches(s)) {
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
+  cfg.stream = s;
+  GIPB_CUDA(cudaLaunchKernelEx(&cfg, k_amg_small<T>, reinterpret_cast<const CycleOp<T>*>(M.small_ops.p),
+                               M.small_nops, S));
+  return GIPB200_OK;
+}
+template int plan_small_levels(AmgT<float>&, cudaStream_t);
+template int plan_small_levels(AmgT<double>&, cudaStream_t);
+template int launch_small_levels(const AmgT<float>&, PcgScalars*, cudaStream_t);
+template int launch_small_levels(const AmgT<double>&, PcgScalars*, cudaStream_t);
 
 // ------------------------------------------------------------------ groups
 int SolveGroups::plan(const std::vector<Pcg*>& solvers, const std::vector<const double*>& b,

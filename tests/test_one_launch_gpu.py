@@ -252,3 +252,28 @@ def test_grouped_batch_solves_equal_the_branches(gpu, monkeypatch, edges):
             assert np.abs(e.field(k) - f.field(k)).max() <= 1e-9 * scale, k
     for k in ("u", "v", "w"):
         assert np.abs(G.instances[0].field(k) - single.field(k)).max() <= 1e-9 * np.abs(single.field("u")).max()
+
+
+@pytest.mark.parametrize("mode,n,fewer", [("mixed", 89, True), ("mixed", 100, True),
+                                          ("tol", 24, True), ("tol", 36, False)])
+def test_small_levels_in_one_launch_are_exact(gpu, monkeypatch, mode, n, fewer):
+    # kernel-by-kernel cycles run their small levels in one launch: every row is summed as its
+    # own kernel sums it, so the steps are the same bit for bit, in fewer kernels (36^3 in FP64
+    # has one level between the finest and the dense one, with more than 1 MB: none)
+    from gip_b200 import cavity
+    from gip_b200.device import DnsEngine
+    case, _ = cavity.generate(n, re=400.0)
+    kw = dict(gamma=1.0 / 400.0, pcg_mode=mode, maxit=2000, tol=1e-8, inner_tol=1e-2,
+              max_outer=100, reorder=True, precond="amg")
+    out = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+        E = DnsEngine(case, **kw)
+        E.advance(2)
+        out.append((E.history()["iters"], E.history()["kernels"], {k: E.field(k) for k in "uvwp"}))
+        E.close()
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.all((out[0][1] < out[1][1]) == fewer)
+    for k in "uvwp":
+        assert np.array_equal(out[0][2][k], out[1][2][k]), k
