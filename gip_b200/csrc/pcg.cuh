@@ -56,14 +56,15 @@ struct CompressedOp {
   double bytes_per_launch = 0.0;     // stored bytes the kernel streams (+ vectors)
 };
 
-// How a whole solve runs as one launch; kNone: kernel by kernel.  kCluster, kGrid, kStream:
-// FP64 with GIP's Jacobi (persist.cu); kSolve: the mixed form and the FP64 tolerance mode
+// How a whole solve runs as one launch; kNone: kernel by kernel.  kBlock, kCluster, kGrid,
+// kStream: FP64 with GIP's Jacobi (persist.cu); kSolve: the mixed form and the FP64 tolerance mode
 // with AMG (persist_amg.cu).
 struct OneLaunch {
-  enum { kNone = 0, kCluster, kGrid, kStream, kSolve };
+  enum { kNone = 0, kBlock, kCluster, kGrid, kStream, kSolve };
   int form = kNone;
   int ctas = 0, threads = 0;
   int per_thread = 1;            // register forms: rows per thread
+  int row_slots = 8;             // block form: longest row
   size_t shared = 0;             // dynamic shared memory per CTA
   DevBuf<double2> pair;          // kGrid, kSolve: (z, p) of every row
   DevBuf<unsigned char> ops;     // kSolve: the V-cycle's products
@@ -151,7 +152,8 @@ struct Pcg {
     if (one.form == OneLaunch::kSolve && counted &&
         (prm.mode == GIPB200_PCG_MIXED) != (prm.precond == GIPB200_PRECOND_AMG))
       return false;
-    return one.form == OneLaunch::kCluster || (one.form != OneLaunch::kNone && !shared_gpu);
+    return one.form == OneLaunch::kBlock || one.form == OneLaunch::kCluster ||
+           (one.form != OneLaunch::kNone && !shared_gpu);
   }
   // scalars and reduction scratch
   DevBuf<PcgScalars> sc;

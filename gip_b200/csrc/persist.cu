@@ -10,6 +10,7 @@
 // with two reductions over all CTAs and no other barrier.  Every row belongs to one thread
 // for the whole solve, which keeps x, r, p, dinv and the row's operator in registers; only
 // the pair (z, p) of a row is ever written, for the threads that gather it.
+//   block form: up to 1920 rows (480 threads, 4 rows each), one CTA; below;
 //   cluster form: up to 16384 rows (16 CTAs of 256 threads, 4 rows each), the pairs in the
 //     cluster's shared memory, the reductions over hardware cluster barriers;
 //   grid form: up to 4 rows per thread of 256 on every SM (151552 rows on 148 SMs), the pairs
@@ -17,8 +18,8 @@
 //   streamed form: more rows, while r and Ap fit the SMs' shared memory (2.1 million rows on
 //     148 SMs), for operators that pack; below.
 // Measured per iteration against the three-kernel loop inside a step graph (host-driven it
-// took 20 us or more): 12^3 2.6 against 12.2 us (cluster of 4; the grid form 4.9), 24^3 4.2
-// (cluster of 16; grid 5.2), 48^3 6.0 against 16.7 (streamed 9.1), 64^3 10.6 against 23
+// took 20 us or more): 8^3 1.4 (block; cluster 2.0), 12^3 2.5 against 12.2 us (block; cluster
+// of 4 2.7; grid 4.9), 24^3 4.2 (cluster of 16; grid 5.2), 48^3 6.0 against 16.7 (streamed 9.1), 64^3 10.6 against 23
 // (host-driven), 128^3 32.5 against 84.
 // Element operations are GIP's (no FMA contraction); only the order of the dot products' sums
 // differs from the other forms.  Columns of ghost cells hold stored zeros in these operators
@@ -53,6 +54,7 @@ struct Args64 {
 // The solve's scalars, held identically by every thread.
 struct Scal64 {
   double rz, pAp, alpha, beta, rr, bb;
+  double goal;  // tol sqrt(b.b), what sqrt(r.r) is compared with
   int iter, done, status;
 };
 
@@ -66,7 +68,8 @@ __device__ __forceinline__ void start64(Scal64& T, const double (&t)[3], int mod
   T.iter = 0;
   T.status = GIPB200_OK;
   T.done = (maxit <= 0) ? 1 : 0;
-  if (mode == GIPB200_PCG_TOL && !(sqrt(t[1]) > tol * sqrt(t[2]))) T.done = 1;
+  T.goal = mode == GIPB200_PCG_TOL ? tol * sqrt(t[2]) : 0.0;
+  if (mode == GIPB200_PCG_TOL && !(sqrt(t[1]) > T.goal)) T.done = 1;
   if (mode != GIPB200_PCG_FIXED && !(isfinite(t[1]) && isfinite(t[2]))) {
     T.status = GIPB200_ERR_BREAKDOWN;
     T.done = 1;
@@ -86,14 +89,13 @@ __device__ __forceinline__ bool alpha64(Scal64& T, double pAp, int mode) {
 }
 
 // After r.z and r.r.
-__device__ __forceinline__ void beta64(Scal64& T, const double (&t)[2], int mode, int maxit,
-                                       double tol) {
+__device__ __forceinline__ void beta64(Scal64& T, const double (&t)[2], int mode, int maxit) {
   const double r0 = T.rz;
   T.rz = t[0];
   T.rr = t[1];
   T.beta = ddiv(t[0], r0);
   T.iter += 1;
-  if (mode == GIPB200_PCG_TOL && !(sqrt(t[1]) > tol * sqrt(T.bb))) T.done = 1;
+  if (mode == GIPB200_PCG_TOL && !(sqrt(t[1]) > T.goal)) T.done = 1;
   if (T.iter >= maxit) {
     if (mode == GIPB200_PCG_TOL && !T.done) T.status = GIPB200_ERR_NOT_CONVERGED;
     T.done = 1;
@@ -147,8 +149,7 @@ struct ClusterPairs {
       if (lane < (int)size)
         st_cluster(map_shared(smem_u32(&red[par][k][rank * nw + warp]), (unsigned)lane), t);
     }
-    if (size == 1u) __syncthreads();  // (a cluster barrier costs 370 cycles, this 30)
-    else cluster_barrier();
+    cluster_barrier();
     const int total = nw * (int)size;
 #pragma unroll
     for (int k = 0; k < W; ++k) {
@@ -253,7 +254,7 @@ __device__ __forceinline__ void solve_rows(const Args64& A, Pairs& Q, int rank, 
       x[k] = dadd(x[k], dmul(T.alpha, p[k]));
     }
     if (!(ok = Q.template sum<2, true>(e))) break;
-    beta64(T, e, A.mode, A.maxit, A.tol);
+    beta64(T, e, A.mode, A.maxit);
   }
 #pragma unroll
   for (int k = 0; k < K; ++k)
@@ -286,6 +287,124 @@ __global__ void __launch_bounds__(kRegThreads, 1) k_pcg64_grid(const __grid_cons
   Q.pairs = A.pair;
   Q.G = grid_begin(A.slots);
   solve_rows<K>(A, Q, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// ------------------------------------------------------------------ block form
+// Small systems in one CTA: p in shared memory, a row's operator in its thread's registers
+// (columns as 16-bit rows), no cluster barriers (370 cycles each) and no remote gathers, at the
+// price of one more block barrier (30 to 60 cycles), between the update of p and its gathers.
+// Few warps with up to four rows a thread: the shuffles of the reductions, an instruction a
+// cycle for the whole SM, would bound a CTA of 1024 threads.  One thread keeps the scalars.
+constexpr int kBlockThreads = 480;  // 128 registers a thread, 48 KB for four rows each
+
+// Sums over the CTA; the first thread of the CTA receives them (finish), before a barrier.
+template <int W, class F>
+__device__ __forceinline__ void block_sum(double (&v)[W], double (*part)[kBlockThreads / 32], F finish) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    const double t = warp_reduce<SumOp>(v[k]);
+    if (lane == 0) part[k][warp] = t;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double t[W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) t[k] = warp_reduce<SumOp>(lane < nw ? part[k][lane] : 0.0);
+    if (lane == 0) finish(t);
+  }
+  __syncthreads();
+}
+
+// K rows per thread of at most SLOTS entries.
+template <int K, int SLOTS>
+__global__ void __launch_bounds__(kBlockThreads, 1) k_pcg64_block(const __grid_constant__ Args64 A) {
+  constexpr bool kLean = K > 2;  // x and dinv in shared memory: registers
+  __shared__ double sp[K * kBlockThreads];
+  __shared__ double sx[kLean ? K * kBlockThreads : 1], sd[kLean ? K * kBlockThreads : 1];
+  __shared__ double part[3][kBlockThreads / 32];
+  __shared__ Scal64 T;
+  const int lane = threadIdx.x & 31, nt = blockDim.x;
+  unsigned at[K][(SLOTS + 1) / 2];  // two columns a word
+  double v[K][SLOTS];
+  double xr[kLean ? 1 : K], dr[kLean ? 1 : K], r[K], z[K], p[K], q[K];
+  auto X = [&](int k) -> double& { return kLean ? sx[k * nt + (int)threadIdx.x] : xr[kLean ? 0 : k]; };
+  auto D = [&](int k) -> double& { return kLean ? sd[k * nt + (int)threadIdx.x] : dr[kLean ? 0 : k]; };
+  double acc3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = k * nt + (int)threadIdx.x;
+    const bool own = i < A.n;
+    long long base = 0;
+    int len = 0;
+    const int s = i >> 5;
+    if (s < A.L.nslices) slice_range(A.L, s, base, len);
+    double sum = 0.0;
+#pragma unroll
+    for (int j = 0; j < (SLOTS + 1) / 2; ++j) at[k][j] = 0u;
+#pragma unroll
+    for (int j = 0; j < SLOTS; ++j) {
+      const int c = (j < len) ? A.L.col[base + 32LL * j + lane] : -1;
+      v[k][j] = (c >= 0) ? A.L.val[base + 32LL * j + lane] : 0.0;
+      if (c >= 0) sum = dadd(sum, dmul(A.x0[c], v[k][j]));
+      // padding and ghost columns: the row's own p times a zero
+      at[k][j / 2] |= (unsigned)((c >= 0 && c < A.n) ? c : (own ? i : 0)) << (16 * (j & 1));
+    }
+    r[k] = z[k] = p[k] = q[k] = 0.0;
+    X(k) = 0.0;
+    D(k) = 0.0;
+    if (own) {
+      const double bi = A.b[i];
+      X(k) = A.x0[i];
+      D(k) = A.dinv[i];
+      r[k] = dadd(bi, dmul(-1.0, sum));
+      z[k] = dadd(0.0, dmul(r[k], D(k)));
+      acc3[0] = dadd(acc3[0], dmul(r[k], z[k]));
+      acc3[1] = dadd(acc3[1], dmul(r[k], r[k]));
+      acc3[2] = dadd(acc3[2], dmul(bi, bi));
+    }
+  }
+  block_sum(acc3, part, [&](const double (&t)[3]) { start64(T, t, A.mode, A.maxit, A.tol); });
+  if (A.x != A.x0)  // (after the reduction: every row has read x0)
+    for (int g = A.n + (int)threadIdx.x; g < A.n_all; g += nt) A.x[g] = A.x0[g];
+  while (!T.done) {
+    const double beta = T.beta;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      p[k] = dadd(z[k], dmul(beta, p[k]));
+      sp[k * nt + (int)threadIdx.x] = p[k];
+    }
+    __syncthreads();
+    double d[1] = {0.0};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      double pv[SLOTS];
+#pragma unroll
+      for (int j = 0; j < SLOTS; ++j) pv[j] = sp[(at[k][j / 2] >> (16 * (j & 1))) & 0xffffu];
+      double sum = 0.0;
+#pragma unroll
+      for (int j = 0; j < SLOTS; ++j) sum = dadd(sum, dmul(pv[j], v[k][j]));
+      q[k] = sum;
+      d[0] = dadd(d[0], dmul(p[k], q[k]));  // (a thread without a row adds zeros)
+    }
+    block_sum(d, part, [&](const double (&t)[1]) { alpha64(T, t[0], A.mode); });
+    if (T.done) break;  // breakdown
+    const double alpha = T.alpha, malpha = dmul(-1.0, alpha);
+    double e[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      r[k] = dadd(r[k], dmul(malpha, q[k]));
+      z[k] = dadd(0.0, dmul(r[k], D(k)));
+      e[0] = dadd(e[0], dmul(r[k], z[k]));
+      e[1] = dadd(e[1], dmul(r[k], r[k]));
+      X(k) = dadd(X(k), dmul(alpha, p[k]));
+    }
+    block_sum(e, part, [&](const double (&t)[2]) { beta64(T, t, A.mode, A.maxit); });
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (k * nt + (int)threadIdx.x < A.n) A.x[k * nt + (int)threadIdx.x] = X(k);
+  if (threadIdx.x == 0) store64(A.S, T);
 }
 
 // ------------------------------------------------------------------ streamed form
@@ -434,7 +553,7 @@ __global__ void __launch_bounds__(1024, 1) k_pcg64_stream(const __grid_constant_
       e[1] = dadd(e[1], dmul(ri, ri));
     }
     if (!(ok = grid_sum<2, false>(e, G))) break;
-    beta64(T, e, A.mode, A.maxit, A.tol);
+    beta64(T, e, A.mode, A.maxit);
     // C: x += alpha p; p = z + beta p (not after the last iteration)
     if (T.done) {
 #pragma unroll 4
@@ -595,18 +714,28 @@ int Pcg::plan_one_launch(cudaStream_t s) {
   DeviceInfo di;
   GIPB_TRY(device_info(&di));
   const int ctas = std::min(di.nsm, kGridCtasMax);
+  // One CTA as far as its threads hold the rows; above, a second SM's arithmetic is worth the
+  // cluster's barriers (12^3 2.45 against 2.66 us per iteration, but 1.9 / 2.5 at 11^3 and
+  // 1.4 / 2.0 at 8^3).
+  if (longest <= kRowSlots && n <= 4 * kBlockThreads) {
+    one.form = OneLaunch::kBlock;
+    one.per_thread = (n + kBlockThreads - 1) / kBlockThreads;
+    one.row_slots = longest;
+    one.ctas = 1;
+    one.threads = ((n + one.per_thread - 1) / one.per_thread + 31) / 32 * 32;
+    return GIPB200_OK;
+  }
   if (longest <= kRowSlots && n <= kRegThreads * 4 * ClusterPairs::kMaxCtas) {
     // the fewest CTAs that leave a thread at most 4 rows, fewer rows while 8 CTAs (the
     // portable cluster size) hold them
-    int k = n <= kRegThreads ? 1 : n <= kRegThreads * 2 * 8 ? 2 : 4;
+    const int k = n <= kRegThreads * 2 * 8 ? 2 : 4;
     int c = 1;
     while (c * kRegThreads * k < n) c *= 2;
     one.ctas = c;
     one.per_thread = k;
     one.threads = ((n + c * k - 1) / (c * k) + 31) / 32 * 32;
-    const bool fits = k == 1   ? cluster_fits(k_pcg64_cluster<1>, one)
-                      : k == 2 ? cluster_fits(k_pcg64_cluster<2>, one)
-                               : cluster_fits(k_pcg64_cluster<4>, one);
+    const bool fits = k == 2 ? cluster_fits(k_pcg64_cluster<2>, one)
+                             : cluster_fits(k_pcg64_cluster<4>, one);
     if (fits) {
       one.form = OneLaunch::kCluster;
       return GIPB200_OK;
@@ -636,6 +765,14 @@ int Pcg::plan_one_launch(cudaStream_t s) {
 }
 
 namespace {
+template <int K>
+int launch_block(const OneLaunch& o, const Args64& A, cudaStream_t s) {
+  if (o.row_slots <= 7) k_pcg64_block<K, 7><<<1, o.threads, 0, s>>>(A);
+  else k_pcg64_block<K, 8><<<1, o.threads, 0, s>>>(A);
+  GIPB_LAUNCH_CHECK();
+  return GIPB200_OK;
+}
+
 template <class K, class... Args>
 int launch_one(K kern, const OneLaunch& o, cudaStream_t s, const Args&... args) {
   cudaLaunchConfig_t cfg;
@@ -658,14 +795,18 @@ int Pcg::enqueue_one_launch(const double* b, double* x, const double* x0, cudaSt
   Args64 A{L->view(), b, x0, dinv.p, x, one.pair.p, one.slots.p, sc.p, prm.tol, n, n_all,
            prm.mode, prm.maxit};
   launches += 1;
-  if (one.form != OneLaunch::kCluster)
+  if (one.form != OneLaunch::kBlock && one.form != OneLaunch::kCluster)
     GIPB_CUDA(cudaMemsetAsync(one.slots.p, 0, one.slots.n * sizeof(ulonglong2), s));
   const int k = one.per_thread;
   switch (one.form) {
+    case OneLaunch::kBlock:
+      return k == 1   ? launch_block<1>(one, A, s)
+             : k == 2 ? launch_block<2>(one, A, s)
+             : k == 3 ? launch_block<3>(one, A, s)
+                      : launch_block<4>(one, A, s);
     case OneLaunch::kCluster:
-      return k == 1   ? launch_one(k_pcg64_cluster<1>, one, s, A)
-             : k == 2 ? launch_one(k_pcg64_cluster<2>, one, s, A)
-                      : launch_one(k_pcg64_cluster<4>, one, s, A);
+      return k == 2 ? launch_one(k_pcg64_cluster<2>, one, s, A)
+                    : launch_one(k_pcg64_cluster<4>, one, s, A);
     case OneLaunch::kGrid:
       return k == 1   ? launch_one(k_pcg64_grid<1>, one, s, A)
              : k == 2 ? launch_one(k_pcg64_grid<2>, one, s, A)

@@ -277,3 +277,33 @@ def test_small_levels_in_one_launch_are_exact(gpu, monkeypatch, mode, n, fewer):
     assert np.all((out[0][1] < out[1][1]) == fewer)
     for k in "uvwp":
         assert np.array_equal(out[0][2][k], out[1][2][k]), k
+
+
+@pytest.mark.parametrize("wide", [False, True])  # rows of at most six and of eight entries
+@pytest.mark.parametrize("n", [480, 481, 960, 961, 1440, 1441, 1920, 1921])
+def test_block_form_matches_oracle_at_its_edges(gpu, oracle_mod, n, wide):
+    # the one-CTA form at one to four rows a thread, and the first size past it; the solver's
+    # parity bar (1e-10 of the solution's scale)
+    import scipy.sparse as sp
+    from gip_b200 import device as dv
+    n_all = n + 40
+    L = _band(n, n_all, far=50, seed=n)
+    if wide:
+        M = sp.csr_matrix((L.val, L.col, L.rowptr), shape=(n, n_all)).tolil()
+        for i in (0, 50, 100):  # rows with a far coupling, and the last ones with ghost columns
+            for j in (i + 5, i + 9):
+                M[i, j] = M[j, i] = -0.25
+        M = M.tocsr()
+        M.sort_indices()
+        L = Csr(n, n_all, M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data)
+    assert np.diff(L.rowptr).max() == (8 if wide else 6)
+    rng = np.random.default_rng(n)
+    b, x0 = rng.standard_normal(n), rng.standard_normal(n_all)
+    for mode, kw in (("fixed", dict(maxit=9)), ("tol", dict(maxit=500, tol=1e-9))):
+        xr, it, _ = oracle_mod.pcg(L, b, x0, mode=0 if mode == "fixed" else 1, **kw)
+        S = dv.PcgSolver(dv.DeviceMatrix(L), n_all=n_all, mode=mode, **kw)
+        x = _t(np.zeros(n_all))
+        res = S.solve(_t(b), x, _t(x0))
+        assert res["status"] == 0 and abs(res["iterations"] - it) <= 1
+        if res["iterations"] == it:
+            _close(x.cpu().numpy(), xr)
