@@ -651,8 +651,11 @@ bool stream_fits(K kern, size_t shared) {
       cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
       cudaFuncGetAttributes(&fa, kern) != cudaSuccess)
     return false;
-  return shared + fa.sharedSizeBytes <= (size_t)most &&
-         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) ==
+  // the limit belongs to the kernel, not to this solver: always the device's, so that planning
+  // one solver never lowers it below what another launches with
+  const int limit = most - (int)fa.sharedSizeBytes;
+  return shared <= (size_t)std::max(limit, 0) &&
+         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) ==
              cudaSuccess;
 }
 

@@ -307,3 +307,21 @@ def test_block_form_matches_oracle_at_its_edges(gpu, oracle_mod, n, wide):
         assert res["status"] == 0 and abs(res["iterations"] - it) <= 1
         if res["iterations"] == it:
             _close(x.cpu().numpy(), xr)
+
+
+@pytest.mark.parametrize("first,second", [(400000, 160001), (160001, 400000)])
+def test_streamed_solvers_of_different_sizes_live_side_by_side(gpu, oracle_mod, first, second):
+    # each plans its own shared memory on the same kernel: both still launch afterwards, in
+    # either order of creation
+    from gip_b200 import device as dv
+    made = []
+    for n in (first, second):
+        L = _band(n, n, seed=n)
+        b = np.random.default_rng(n).standard_normal(n)
+        S = dv.PcgSolver(dv.DeviceMatrix(L), mode="fixed", maxit=5)
+        made.append((n, S, b, oracle_mod.pcg(L, b, np.zeros(n), maxit=5, mode=0)[0]))
+    for _ in range(2):
+        for n, S, b, xr in made:
+            x = _t(np.zeros(n))
+            assert S.solve(_t(b), x, _t(np.zeros(n)))["iterations"] == 5
+            _close(x.cpu().numpy(), xr)
