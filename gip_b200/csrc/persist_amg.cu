@@ -1310,9 +1310,9 @@ int Pcg::plan_solve_launch(cudaStream_t s) {
   const bool mixed = prm.mode == GIPB200_PCG_MIXED, with_amg = prm.precond == GIPB200_PRECOND_AMG;
   // Where the lines lie (us per iteration, one launch against kernel by kernel, host-driven;
   // in the engine's graph the mixed AMG iteration took 75 at 63^3):
-  //   mixed AMG    63^3 63 / 131, 75^3 75 / 150, 128^3 244 / 189 (dependent launches)
-  //   FP64 AMG     33^3 36 / 94, 63^3 56 / 135, 128^3 276 / 368, 200^3 1004 / 1061
-  //   mixed Jacobi 33^3 8 / 23, 75^3 11 / 28, 128^3 32 / 45, 160^3 73 / 66
+  //   mixed AMG    63^3 63 / 131, 75^3 73 / 150, 128^3 244 / 189 (dependent launches)
+  //   FP64 AMG     33^3 35 / 94, 63^3 57 / 135, 128^3 275 / 368, 200^3 1004 / 1061
+  //   mixed Jacobi 33^3 8 / 23, 75^3 11 / 28, 128^3 34 / 45, 160^3 73 / 66
   // beyond them the 16 to 32 warps a resident CTA leaves per SM gather slower than the 64 of
   // the separate kernels.
   const int most = mixed && with_amg ? 700000 : 2500000;
