@@ -755,6 +755,7 @@ int gipb200_matrix_spmv_values(gipb200_matrix A, const double* x, gipb200_matrix
     int b;
     GIPB_TRY(grid_blocks(256, T->S.nnz, 4, 0, &b));
     T->S.version += 1;
+    T->S.values_in_graph = T->S.values_in_graph || !dependent_launches(s);
     T->P.bits = 0;  // its table holds the old values
     k_scatter_vals<<<b, 256, 0, s>>>(T->S.nnz, T->S.pos.p, T->S.csr_val.p, T->S.val.p);
     GIPB_LAUNCH_CHECK();

@@ -175,7 +175,10 @@ struct Sell {
   int nrows = 0, ncols = 0, nnz = 0, nslices = 0;
   long long nslots = 0;
   bool rows_nonempty = true;  // no empty row
-  unsigned version = 0;       // counts changes of the values (layouts packed from them lapse)
+  // changes of the values after the operator was built: calls that changed them, and whether
+  // one of them was captured (a graph then changes them at any later time, unseen by the host)
+  unsigned version = 0;
+  bool values_in_graph = false;
   int uslots = 0;             // > 0: every slice has this many slots
   DevBuf<long long> sptr;
   DevBuf<int> col;

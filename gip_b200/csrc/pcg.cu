@@ -1367,10 +1367,7 @@ static int host_poll_interval() {
 }
 
 int Pcg::enqueue(const double* b, double* x, const double* x0, cudaStream_t s, bool host_sync) {
-  if (op64.bits && L->version != packed_version) {  // L's values changed since they were packed
-    op64.bits = 0;
-    if (one.form == OneLaunch::kStream || one.form == OneLaunch::kSolve) one.form = OneLaunch::kNone;
-  }
+  follow_values();
   if (one_launch()) return enqueue_one_launch(b, x, x0, s);
   if (!host_sync && prm.mode != GIPB200_PCG_FIXED && capturing(s)) {
     if (!body_stream[0]) {
@@ -1689,6 +1686,7 @@ int Pcg::time_update(int reps, cudaStream_t s, double* avg_ms, double* bytes) {
 
 int Pcg::time_spmv(int mixed, int reps, cudaStream_t s, double* avg_ms, double* bytes) {
   if (reps <= 0) return fail(GIPB200_ERR_ARG, "reps must be positive");
+  follow_values();
   if (mixed && prm.mode != GIPB200_PCG_MIXED)
     return fail(GIPB200_ERR_STATE, "the FP32 kernel exists only in the mixed form");
   if (!mixed && prm.mode == GIPB200_PCG_MIXED)
@@ -1879,6 +1877,12 @@ int gipb200_pcg_get_info(gipb200_pcg S, gipb200_pcg_info* info) {
   info->amg_complexity = amg ? amg->op_complexity : amg64 ? amg64->op_complexity : 0.0;
   info->amg_setup_s = amg ? amg->setup_s : amg64 ? amg64->setup_s : 0.0;
   info->packed_residual = S->P.lpacked ? 1 : 0;
+  return GIPB200_OK;
+}
+
+int gipb200_pcg_solve_form(gipb200_pcg S, int* form) {
+  if (!S || !form) return fail(GIPB200_ERR_ARG, "null argument");
+  *form = S->P.solve_form();
   return GIPB200_OK;
 }
 

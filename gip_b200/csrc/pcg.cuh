@@ -139,8 +139,8 @@ struct Pcg {
   // constant mode is restored exactly from the pin equation.
   int pin_row = -1;
   double pin_val = 0.0;
-  Packed64 op64;                 // L packed (bits = 0: not), at this version of its values
-  unsigned packed_version = 0;
+  Packed64 op64;                 // L packed (bits = 0: not)
+  unsigned planned_version = 0;  // of L's values, when op64 and `one` were made from them
   OneLaunch one;
   // several solvers advance side by side on one GPU (a batch): forms that claim every SM at
   // once (the cooperative ones) would take turns, so only the cluster form runs
@@ -155,6 +155,7 @@ struct Pcg {
     return one.form == OneLaunch::kBlock || one.form == OneLaunch::kCluster ||
            (one.form != OneLaunch::kNone && !shared_gpu);
   }
+  int solve_form();  // GIPB200_SOLVE_* of the next solve
   // scalars and reduction scratch
   DevBuf<PcgScalars> sc;
   DevBuf<double> partials;
@@ -190,6 +191,7 @@ struct Pcg {
 
  private:
   int build_packed64(cudaStream_t s);
+  void follow_values();
   int plan_one_launch(cudaStream_t s);
   int plan_solve_launch(cudaStream_t s);
   int enqueue_solve_launch(const double* b, double* x, const double* x0, cudaStream_t s);

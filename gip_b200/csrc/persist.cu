@@ -632,9 +632,16 @@ __global__ void __launch_bounds__(256, 8) k_pcg64_spmv_dot(SellView<double> L, S
 }  // namespace
 
 // ------------------------------------------------------------------ set-up
-int Pcg::build_packed64(cudaStream_t s) {
-  packed_version = L->version;
-  return pack64(*L, n, false, &op64, s);
+int Pcg::build_packed64(cudaStream_t s) { return pack64(*L, n, false, &op64, s); }
+
+// L's values changed since they were looked at: the FP64 solves read them as they are now, as
+// the kernel-by-kernel loop does.  What was made from the old ones lapses for good: the packed
+// copy, and with ghost columns every form that drops them because they held zeros.  (The mixed
+// form keeps its own copies of L's values, in one launch and kernel by kernel alike.)
+void Pcg::follow_values() {
+  if (prm.mode == GIPB200_PCG_MIXED || (L->version == planned_version && !L->values_in_graph)) return;
+  if (op64.bits || n_all > n) one.form = OneLaunch::kNone;
+  op64.bits = 0;
 }
 
 namespace {
@@ -703,9 +710,22 @@ int Pcg::ghosts_zero(cudaStream_t s, bool* zero) const {
   return GIPB200_OK;
 }
 
+int Pcg::solve_form() {
+  follow_values();
+  if (!one_launch()) return GIPB200_SOLVE_LOOP;
+  switch (one.form) {
+    case OneLaunch::kBlock: return GIPB200_SOLVE_BLOCK;
+    case OneLaunch::kCluster: return GIPB200_SOLVE_CLUSTER;
+    case OneLaunch::kGrid: return GIPB200_SOLVE_GRID;
+    case OneLaunch::kStream: return GIPB200_SOLVE_STREAM;
+    default: return one.cluster ? GIPB200_SOLVE_PRECOND_CLUSTER : GIPB200_SOLVE_PRECOND_GRID;
+  }
+}
+
 // Which one-launch form runs this solver's solves.
 int Pcg::plan_one_launch(cudaStream_t s) {
   one.form = OneLaunch::kNone;
+  planned_version = L->version;
   if (prm.mode == GIPB200_PCG_MIXED || prm.precond != GIPB200_PRECOND_JACOBI)
     return plan_solve_launch(s);
   if (n <= 0 || !L->rows_nonempty || getenv("GIPB200_NO_ONE_LAUNCH")) return GIPB200_OK;

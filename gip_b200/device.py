@@ -177,6 +177,8 @@ def pcg_params(mode: str = "fixed", maxit: int = 100, tol: float = 1e-6,
                        PRECONDS[precond])
 
 
+# how a solve runs (GIPB200_SOLVE_*)
+SOLVE_FORMS = ("loop", "block", "cluster", "grid", "stream", "precond_cluster", "precond_grid")
 CYCLE_KINDS = ("jacobi0", "residual", "restrict", "dense", "prolong", "smooth", "tail")
 # the kernel each product form runs as (GIPB200_FORM_*)
 FORM_KERNELS = ("k_amgp_spmv", "k_amg_spmv", "k_amg_spmv_pf", "k_amg_csr", "k_amg_dense",
@@ -236,6 +238,12 @@ class PcgSolver:
         L.call("gipb200_pcg_kernel_time", self.handle, reps, _stream(stream), C.byref(ms),
                C.byref(nb))
         return ms.value, nb.value
+
+    def solve_form(self) -> str:
+        """How the next solve runs: "loop" (kernel by kernel) or its one-launch form."""
+        f = C.c_int()
+        L.call("gipb200_pcg_solve_form", self.handle, C.byref(f))
+        return SOLVE_FORMS[f.value]
 
     def info(self) -> dict:
         i = L.PcgInfo()

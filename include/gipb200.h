@@ -211,6 +211,18 @@ typedef struct {
   int packed_residual;         /* MIXED: FP64 residual from the packed columns (1) or L   */
 } gipb200_pcg_info;
 int gipb200_pcg_get_info(gipb200_pcg S, gipb200_pcg_info* info);
+/* No counterpart in the reference: how the solver's next solve runs (GIPB200_SOLVE_*): kernel
+ * by kernel, or as one launch over one thread block, a thread-block cluster or every SM. */
+enum {
+  GIPB200_SOLVE_LOOP = 0,      /* kernel by kernel                                        */
+  GIPB200_SOLVE_BLOCK = 1,     /* FP64 Jacobi, one block                                  */
+  GIPB200_SOLVE_CLUSTER = 2,   /* FP64 Jacobi, one cluster                                */
+  GIPB200_SOLVE_GRID = 3,      /* FP64 Jacobi, cooperative grid, state in registers       */
+  GIPB200_SOLVE_STREAM = 4,    /* FP64 Jacobi, cooperative grid, packed operator streamed */
+  GIPB200_SOLVE_PRECOND_CLUSTER = 5, /* MIXED, or TOL with AMG: one cluster               */
+  GIPB200_SOLVE_PRECOND_GRID = 6     /* MIXED, or TOL with AMG: cooperative grid          */
+};
+int gipb200_pcg_solve_form(gipb200_pcg S, int* form);
 /* No counterpart in the reference: times `reps` launches of the solver's SpMV-dot kernel
  * (FP64 forms: the FP64 kernel; MIXED: the FP32 kernel of its operator layout) on its
  * current search direction, with CUDA events on `stream`; returns the mean launch time and
