@@ -730,7 +730,7 @@ int gipb200_matrix_info(gipb200_matrix A, int* nrows, int* ncols, int* nnz, int6
 int gipb200_matrix_spmv(gipb200_matrix A, const double* x, double* y, double alpha, double beta,
                         int mode, void* stream) {
   if (!A || (mode != 0 && mode != 1)) return fail(GIPB200_ERR_ARG, "null matrix or bad mode");
-  if (A->P.bits)
+  if (packed_product(*A, as_stream(stream)))
     return launch_packed_spmv(A->S, A->P, x, y, alpha, beta, mode, as_stream(stream));
   return launch_sell_spmv(A->S, A->S.val.p, x, y, alpha, beta, mode, as_stream(stream));
 }

@@ -152,7 +152,7 @@ int gipb200_matrix_spmv_dot(gipb200_matrix A, const double* d_x, double* d_y, in
     return fail(GIPB200_ERR_ARG, "spmv_dot: n_dot=%d outside [0, rows=%d]", n_dot, A->S.nrows);
   if (d_x == d_y) return fail(GIPB200_ERR_ARG, "spmv_dot: x and y must not alias");
   cudaStream_t s = as_stream(stream);
-  if (A->P.bits && A->S.nrows > 0)
+  if (A->S.nrows > 0 && packed_product(*A, s))
     return launch_packed_spmv_dot(A->S, A->P, d_x, d_y, n_dot, A->rs, d_dot, s);
   int blocks = 1;
   GIPB_TRY(grid_blocks(256, std::max(A->S.nslices, 1) * 32, 1, kMaxReduceBlocks, &blocks));

@@ -268,3 +268,9 @@ struct gipb200_matrix_s {
   gipb200::DevBuf<unsigned> ticket;
   gipb200::ReduceScratch rs{};
 };
+
+// Whether a product of the handle reads the packed words: they hold the values of now, while
+// a captured product must read those of each later replay, which the sliced arrays have.
+inline bool packed_product(const gipb200_matrix_s& A, cudaStream_t s) {
+  return A.P.bits && gipb200::dependent_launches(s);
+}

@@ -80,3 +80,38 @@ def test_forms_without_ghosts_read_new_values(gpu, n, form):
     S.solve(b, x, torch.zeros_like(b))
     dv.PcgSolver(dv.DeviceMatrix(new), **FIXED).solve(b, y, torch.zeros_like(b))
     assert float((x - y).abs().max()) <= 1e-10 * float(y.abs().max())
+
+
+@pytest.mark.parametrize("together", [True, False])
+def test_captured_products_read_the_values_of_their_replay(gpu, together):
+    # a handle large enough for the packed layout: products captured with a later spmv_values
+    # (the second replay's products are the new values'), and products captured alone, replayed
+    # after an spmv_values that was not captured; the products' sums keep their order, bit for bit
+    from gip_b200 import device as dv
+    n = 220000
+    old = _band(n, n, seed=4)
+    new = Csr(n, n, old.rowptr, old.col, np.random.default_rng(1).standard_normal(old.nnz))
+    T = dv.DeviceMatrix(old)
+    eye = dv.DeviceMatrix(Csr(old.nnz, old.nnz, np.arange(old.nnz + 1, dtype=np.int32),
+                              np.arange(old.nnz, dtype=np.int32), np.ones(old.nnz)))
+    v = _t(new.val)
+    x = torch.randn(n, dtype=torch.float64, device="cuda")
+    first = T.spmv(x, torch.zeros_like(x))
+    second = dv.DeviceMatrix(new).spmv(x, torch.zeros_like(x))
+    y, z, d = torch.zeros_like(x), torch.zeros_like(x), x.new_zeros(1)
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        T.spmv(x, y)
+        T.spmv_dot(x, z, d)
+        if together:
+            eye.spmv_values(v, T)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, first) and torch.equal(z, first)
+    if not together:
+        eye.spmv_values(v, T)
+        torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, second) and torch.equal(z, second)
