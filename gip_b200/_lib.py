@@ -148,6 +148,8 @@ _SIGNATURES = {
     "gipb200_dns_destroy": (_I, [_VP]),
     "gipb200_dns_advance": (_I, [_VP, _I, _VP]),
     "gipb200_dns_history": (_I, [_VP, C.POINTER(_I), _VP, _VP, _VP, _VP, _VP, _VP, _VP]),
+    "gipb200_dns_solve_status": (_I, [_VP, _I, _VP, C.POINTER(_I)]),
+    "gipb200_dns_check_bounded_wait": (_I, [_VP, _VP, C.POINTER(_I)]),
     "gipb200_dns_step_phases": (_I, [_VP, _VP, _VP]),
     "gipb200_dns_phase_stamps": (_I, [_VP, _I]),
     "gipb200_amg_host_levels": (_I, [_I, _VP, _VP, _VP, _VP, _I, C.c_double, _I, C.POINTER(_I),

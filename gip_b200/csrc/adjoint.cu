@@ -519,6 +519,7 @@ int gipb200_adjoint_forward(gipb200_adjoint H, const double* h_lid, double nu_sc
     A.E.graph = nullptr;
   }
   GIPB_TRY(A.reset_state(s));
+  A.E.pcg.clear_gave_up();
   // the checkpoints are kept from call to call (their device buffers are reused: a forward
   // allocates only when it needs more segments than the last one)
   const int K = A.prm.checkpoint_every;
@@ -558,7 +559,7 @@ int gipb200_adjoint_forward(gipb200_adjoint H, const double* h_lid, double nu_sc
     GIPB_LAUNCH_CHECK();
   }
   GIPB_CUDA(cudaDeviceSynchronize());
-  return GIPB200_OK;
+  return A.E.check_solves();
 }
 
 int gipb200_adjoint_backward(gipb200_adjoint H, double* h_grad_lid, double* h_grad_nu) {
@@ -582,6 +583,7 @@ int gipb200_adjoint_backward(gipb200_adjoint H, double* h_grad_lid, double* h_gr
     cudaGraphDestroy(A.E.graph);
     A.E.graph = nullptr;
   }
+  A.adj.clear_gave_up();
   // adjoint state after the last step (ub seeded by the forward)
   GIPB_TRY(A.mfb.zero(s));
   for (int d = 0; d < 3; ++d) GIPB_TRY(A.a0b[d].zero(s));
@@ -594,6 +596,9 @@ int gipb200_adjoint_backward(gipb200_adjoint H, double* h_grad_lid, double* h_gr
     for (int n = n1 - 1; n >= n0; --n) GIPB_TRY(A.adjoint_step(n, n - n0, s));
   }
   GIPB_CUDA(cudaDeviceSynchronize());
+  GIPB_TRY(A.E.check_solves());
+  if (A.adj.wait_gave_up())
+    return fail(GIPB200_ERR_TIMEOUT, "a wait of an adjoint Poisson solve gave up");
   if (A.n_lid) {
     DevBuf<double> g;
     GIPB_TRY(g.alloc(A.n_lid));

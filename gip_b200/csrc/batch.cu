@@ -276,6 +276,7 @@ int gipb200_batch_advance(gipb200_batch H, int nsteps, void* stream) {
   cudaStream_t s = as_stream(stream);
   // host-side preparation of every instance: history room, initial dt
   bool recapture = false;
+  for (auto d : B.inst) GIPB_TRY(d->E.check_solves());
   for (auto d : B.inst) {
     Dns& E = d->E;
     const int cap_before = E.capacity;
@@ -386,11 +387,15 @@ int gipb200_batch_solver_status(gipb200_batch H, void* stream, int* h_err) {
   if (!H || !h_err) return fail(GIPB200_ERR_ARG, "null argument");
   Batch& B = H->B;
   *h_err = 0;
-  if (!B.d_err.p) return GIPB200_OK;
   cudaStream_t s = as_stream(stream);
-  GIPB_CUDA(cudaMemcpyAsync(h_err, B.d_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (B.d_err.p)
+    GIPB_CUDA(cudaMemcpyAsync(h_err, B.d_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   GIPB_CUDA(cudaStreamSynchronize(s));
-  GIPB_CUDA(cudaMemsetAsync(B.d_err.p, 0, sizeof(int), s));
+  if (B.d_err.p) GIPB_CUDA(cudaMemsetAsync(B.d_err.p, 0, sizeof(int), s));
+  for (auto d : B.inst) {  // one-launch solves, grouped or in the branches
+    if (d->E.pcg.wait_gave_up()) *h_err = 1;
+    d->E.pcg.clear_gave_up();
+  }
   return GIPB200_OK;
 }
 

@@ -510,6 +510,7 @@ struct CflStepFinish {
         H.dt[k] = S->dt;
         H.iters[k] = pcg_mixed ? P->total_inner : P->iter;
         H.rr[k] = P->rr;
+        H.status[k] = P->status;
         H.outer[k] = pcg_mixed ? P->outer : 0;
         // the step's 10 kernels and the PCG's: init + 3 per iteration in the FP64 forms
         // (2 with AMG, whose V-cycle and direction kernels count themselves on the device),
@@ -561,12 +562,13 @@ int Dns::grow_history(int need, cudaStream_t s) {
   if (need <= capacity) return GIPB200_OK;
   int cap = std::max(need, std::max(1024, capacity * 2));
   DevBuf<double> t, d, m, r;
-  DevBuf<int> it, ou, kn;
+  DevBuf<int> it, ou, kn, ss;
   DevBuf<unsigned long long> st;
   GIPB_TRY(st.alloc((size_t)cap * kPhaseMarks));
   GIPB_CUDA(cudaMemsetAsync(st.p, 0, (size_t)cap * kPhaseMarks * 8, s));
   GIPB_TRY(ou.alloc(cap));
   GIPB_TRY(kn.alloc(cap));
+  GIPB_TRY(ss.alloc(cap));
   GIPB_TRY(t.alloc(cap));
   GIPB_TRY(d.alloc(cap));
   GIPB_TRY(m.alloc(cap));
@@ -580,6 +582,7 @@ int Dns::grow_history(int need, cudaStream_t s) {
     GIPB_CUDA(cudaMemcpyAsync(it.p, h_iters.p, capacity * 4, cudaMemcpyDeviceToDevice, s));
     GIPB_CUDA(cudaMemcpyAsync(ou.p, h_outer.p, capacity * 4, cudaMemcpyDeviceToDevice, s));
     GIPB_CUDA(cudaMemcpyAsync(kn.p, h_kernels.p, capacity * 4, cudaMemcpyDeviceToDevice, s));
+    GIPB_CUDA(cudaMemcpyAsync(ss.p, h_status.p, capacity * 4, cudaMemcpyDeviceToDevice, s));
     GIPB_CUDA(cudaMemcpyAsync(st.p, h_stamps.p, (size_t)capacity * kPhaseMarks * 8,
                               cudaMemcpyDeviceToDevice, s));
   }
@@ -591,14 +594,21 @@ int Dns::grow_history(int need, cudaStream_t s) {
   std::swap(h_iters.p, it.p);
   std::swap(h_outer.p, ou.p);
   std::swap(h_kernels.p, kn.p);
+  std::swap(h_status.p, ss.p);
   std::swap(h_stamps.p, st.p);
-  h_time.n = h_dt.n = h_massr.n = h_rr.n = h_iters.n = h_outer.n = h_kernels.n = cap;
-  t.n = d.n = m.n = r.n = it.n = ou.n = kn.n = capacity;
+  h_time.n = h_dt.n = h_massr.n = h_rr.n = h_iters.n = h_outer.n = h_kernels.n = h_status.n = cap;
+  t.n = d.n = m.n = r.n = it.n = ou.n = kn.n = ss.n = capacity;
   h_stamps.n = (size_t)cap * kPhaseMarks;
   st.n = (size_t)capacity * kPhaseMarks;
   capacity = cap;
   drop_graph();  // a captured graph refers to the old history arrays
   return GIPB200_OK;
+}
+
+int Dns::check_solves() const {
+  if (!pcg.wait_gave_up()) return GIPB200_OK;
+  return fail(GIPB200_ERR_TIMEOUT,
+              "a wait of an earlier step's pressure solve gave up: the state is not valid");
 }
 
 int Dns::enqueue_initial_dt(cudaStream_t s) {
@@ -1265,6 +1275,7 @@ int dns_init(Dns& E, const gipb200_dns_ops* ops, const double* h_u, const double
 }
 
 int dns_advance(Dns& E, int nsteps, cudaStream_t s) {
+  GIPB_TRY(E.check_solves());
   GIPB_TRY(E.grow_history(E.steps_enqueued + nsteps, s));
   if (!E.started) {
     GIPB_TRY(E.enqueue_initial_dt(s));
@@ -1341,6 +1352,7 @@ int gipb200_dns_step_phases(gipb200_dns Dh, void* stream, double* h_ms) {
   if (!Dh || !h_ms) return fail(GIPB200_ERR_ARG, "null argument");
   Dns& E = Dh->E;
   cudaStream_t s = as_stream(stream);
+  GIPB_TRY(E.check_solves());
   GIPB_TRY(E.grow_history(E.steps_enqueued + 1, s));
   if (!E.started) {
     GIPB_TRY(E.enqueue_initial_dt(s));
@@ -1422,6 +1434,23 @@ int gipb200_dns_history(gipb200_dns Dh, int* steps, double* t, double* dt, doubl
   if (outer && n) GIPB_CUDA(cudaMemcpy(outer, E.h_outer.p, n * 4, cudaMemcpyDeviceToHost));
   if (kernels && n) GIPB_CUDA(cudaMemcpy(kernels, E.h_kernels.p, n * 4, cudaMemcpyDeviceToHost));
   return GIPB200_OK;
+}
+
+int gipb200_dns_solve_status(gipb200_dns Dh, int max_steps, int* h_status, int* steps_out) {
+  if (!Dh || max_steps < 0 || (max_steps > 0 && !h_status)) return fail(GIPB200_ERR_ARG, "bad arguments");
+  Dns& E = Dh->E;
+  GIPB_CUDA(cudaDeviceSynchronize());
+  DnsScalars S;
+  GIPB_CUDA(cudaMemcpy(&S, E.sc.p, sizeof(S), cudaMemcpyDeviceToHost));
+  const int n = std::min(std::min(S.step, E.capacity), max_steps);
+  if (steps_out) *steps_out = n;
+  if (n > 0) GIPB_CUDA(cudaMemcpy(h_status, E.h_status.p, (size_t)n * 4, cudaMemcpyDeviceToHost));
+  return GIPB200_OK;
+}
+
+int gipb200_dns_check_bounded_wait(gipb200_dns Dh, void* stream, int* h_status) {
+  if (!Dh || !h_status) return fail(GIPB200_ERR_ARG, "null argument");
+  return Dh->E.pcg.check_bounded_wait(as_stream(stream), h_status);
 }
 
 int gipb200_dns_get_field(gipb200_dns Dh, const char* name, double* h_out, int n) {
@@ -1568,10 +1597,12 @@ int gipb200_dns_snapshot(gipb200_dns Dh, int restore, void* stream) {
   k_copy_state<<<C.first[C.count], StateCopy::kThreads, 0, s>>>(C);
   GIPB_LAUNCH_CHECK();
   E.launches += 1;
-  if (restore)
+  if (restore) {
     E.steps_enqueued = E.snap_steps;
-  else
+    E.pcg.clear_gave_up();
+  } else {
     E.snap_steps = E.steps_enqueued;
+  }
   return GIPB200_OK;
 }
 

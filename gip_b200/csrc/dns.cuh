@@ -22,6 +22,7 @@ struct DnsHistory {
   double* rr;
   int* outer;
   int* kernels;  // kernels the step launched (early exits included)
+  int* status;   // the pressure solve's status
   unsigned long long* stamps;  // kPhaseMarks device times per step (phase stamps on)
   int capacity;
   int stamp_kernels;  // phase-stamp kernels each step adds (0 when stamps are off)
@@ -69,7 +70,7 @@ struct Dns {
   Pcg pcg;
   DevBuf<DnsScalars> sc;
   DevBuf<double> h_time, h_dt, h_massr, h_rr;
-  DevBuf<int> h_iters, h_outer, h_kernels;
+  DevBuf<int> h_iters, h_outer, h_kernels, h_status;
   DevBuf<unsigned long long> h_stamps;  // capacity x kPhaseMarks, 0 = not recorded
   bool stamps_on = false;               // stamp the phase boundaries on the device
   int capacity = 0;
@@ -109,7 +110,7 @@ struct Dns {
   }
   DnsHistory history() const {
     return {h_time.p,    h_dt.p,     h_massr.p, h_iters.p,
-            h_rr.p,      h_outer.p,  h_kernels.p, h_stamps.p,
+            h_rr.p,      h_outer.p,  h_kernels.p, h_status.p, h_stamps.p,
             capacity,    stamps_on ? kPhaseMarks : 0};
   }
   void drop_graph() {
@@ -119,6 +120,8 @@ struct Dns {
     graph = nullptr;
   }
   int grow_history(int need, cudaStream_t s);
+  // Steps after a pressure solve whose wait gave up are refused: the state is not valid.
+  int check_solves() const;
   // Algorithmic bytes of each phase of one timestep, in gipb200_dns_step_phases order
   // (the PCG entry is 0: its bytes are iterations x iteration_bytes + replacements).
   void phase_bytes(double out[7]) const;

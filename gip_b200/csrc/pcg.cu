@@ -828,6 +828,7 @@ __global__ void k_pcg_inv_diag(int nrows, const int* __restrict__ rp, const int*
 // ------------------------------------------------------------------ host side
 Pcg::~Pcg() {
   if (h_sc) cudaFreeHost(h_sc);
+  if (gave_up) cudaFreeHost(gave_up);
   for (auto& bs : body_stream)
     if (bs) cudaStreamDestroy(bs);
 }
@@ -857,6 +858,8 @@ int Pcg::init(const Sell* Lm, int nall, const gipb200_pcg_params& params, cudaSt
   GIPB_TRY(sc.alloc(1));
   GIPB_TRY(sc.zero(s));
   GIPB_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_sc), sizeof(PcgScalars)));
+  GIPB_CUDA(cudaMallocHost(reinterpret_cast<void**>(&gave_up), sizeof(int)));
+  clear_gave_up();
   for (auto& bs : body_stream) GIPB_CUDA(cudaStreamCreateWithFlags(&bs, cudaStreamNonBlocking));
   GIPB_TRY(grid_blocks(256, L->nslices * 32, 1, kMaxReduceBlocks, &blocks_spmv));
   GIPB_TRY(grid_blocks(256, std::max(n, 1), 4, kMaxReduceBlocks, &blocks_vec));

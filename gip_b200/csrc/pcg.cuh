@@ -162,6 +162,16 @@ struct Pcg {
   DevBuf<unsigned> ticket;
   ReduceScratch rs{};
   PcgScalars* h_sc = nullptr;  // pinned
+  // pinned, written by the kernel of a one-launch solve whose wait gave up: x of that solve, and
+  // what was made from it, is not valid
+  int* gave_up = nullptr;
+  bool wait_gave_up() const { return gave_up && *static_cast<volatile int*>(gave_up) != 0; }
+  void clear_gave_up() {
+    if (gave_up) *static_cast<volatile int*>(gave_up) = 0;
+  }
+  // Runs solves and a barrier that wait for a CTA that does not exist, on this solver's scalars
+  // and flag; *status = GIPB200_ERR_TIMEOUT when each gave up and said so.
+  int check_bounded_wait(cudaStream_t s, int* status);
   int blocks_spmv = 1, blocks_vec = 1;
   // launch shape overrides (autotuning): 0 = default grid
   int set_launch(int spmv_blocks, int vec_blocks);
@@ -195,6 +205,7 @@ struct Pcg {
   int plan_one_launch(cudaStream_t s);
   int plan_solve_launch(cudaStream_t s);
   int enqueue_solve_launch(const double* b, double* x, const double* x0, cudaStream_t s);
+  void launch_wait_check(bool barrier_only, ulonglong2* slots, cudaStream_t s);
   int ghosts_zero(cudaStream_t s, bool* zero) const;  // L's ghost columns all hold 0.0
   void launch_packed64_spmv(double* q, PcgScalars* S, int mode, cudaStream_t s);
   // operator bytes a product streams from the packed FP64 layout: column deltas, value

@@ -47,6 +47,7 @@ struct Args64 {
   double2* pair;      // grid form: (z, p) of every row
   ulonglong2* slots;  // grid forms: reduction slots (zero at launch)
   PcgScalars* S;
+  int* gave_up;       // host flag: a wait gave up
   double tol;
   int n, n_all, mode, maxit;
 };
@@ -114,6 +115,15 @@ __device__ __forceinline__ void store64(PcgScalars* S, const Scal64& T) {
   S->status = T.status;
   S->kernels = 0;
   S->one_launch = 1;
+}
+
+// The end of a solve over several CTAs (one thread of each).
+__device__ __forceinline__ void finish64(const Args64& A, Scal64& T, int rank, bool ok) {
+  if (!ok) {
+    T.status = GIPB200_ERR_TIMEOUT;
+    report_gave_up(A.gave_up);
+  }
+  if (rank == 0) store64(A.S, T);
 }
 
 // ------------------------------------------------------------------ register forms
@@ -259,8 +269,7 @@ __device__ __forceinline__ void solve_rows(const Args64& A, Pairs& Q, int rank, 
 #pragma unroll
   for (int k = 0; k < K; ++k)
     if (i0 + k * (int)blockDim.x < A.n) A.x[i0 + k * (int)blockDim.x] = x[k];
-  if (!ok) T.status = GIPB200_ERR_TIMEOUT;
-  if (rank == 0 && threadIdx.x == 0) store64(A.S, T);
+  if (threadIdx.x == 0) finish64(A, T, rank, ok);
 }
 
 constexpr int kRegThreads = 256;  // CTA size of the register forms
@@ -287,6 +296,15 @@ __global__ void __launch_bounds__(kRegThreads, 1) k_pcg64_grid(const __grid_cons
   Q.pairs = A.pair;
   Q.G = grid_begin(A.slots);
   solve_rows<K>(A, Q, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// One CTA of a group that claims two and has no rows: its first sum waits for a CTA that does
+// not exist and gives up.
+__global__ void __launch_bounds__(kRegThreads, 1) k_pcg64_wait_check(const __grid_constant__ Args64 A) {
+  GridPairs Q;
+  Q.pairs = A.pair;
+  Q.G = grid_begin(A.slots, 0, 2, kCheckSpinCycles);
+  solve_rows<1>(A, Q, 0, 1);
 }
 
 // ------------------------------------------------------------------ block form
@@ -570,8 +588,7 @@ __global__ void __launch_bounds__(1024, 1) k_pcg64_stream(const __grid_constant_
     double none[1] = {0.0};
     ok = grid_sum<1, true>(none, G);
   }
-  if (!ok) T.status = GIPB200_ERR_TIMEOUT;
-  if (rank == 0 && threadIdx.x == 0) store64(A.S, T);
+  if (threadIdx.x == 0) finish64(A, T, rank, ok);
 }
 
 struct AlphaFinish64 {
@@ -807,6 +824,29 @@ int launch_one(K kern, const OneLaunch& o, cudaStream_t s, const Args&... args) 
 }
 }  // namespace
 
+// The FP64 register form and the preconditioned form (persist_amg.cu), one after the other.
+int Pcg::check_bounded_wait(cudaStream_t s, int* status) {
+  DevBuf<ulonglong2> slots;
+  GIPB_TRY(slots.alloc(grid_slot_count(2)));
+  Args64 A{};
+  A.slots = slots.p;
+  A.S = sc.p;
+  A.gave_up = gave_up;
+  A.maxit = 1;
+  *status = GIPB200_ERR_TIMEOUT;
+  for (int k = 0; k < 3; ++k) {
+    GIPB_TRY(slots.zero(s));
+    GIPB_TRY(sc.zero(s));
+    clear_gave_up();
+    if (k == 0) k_pcg64_wait_check<<<1, kRegThreads, 0, s>>>(A);
+    else launch_wait_check(k == 2, slots.p, s);
+    GIPB_LAUNCH_CHECK();
+    GIPB_TRY(result(s, nullptr));
+    if (h_sc->status != GIPB200_ERR_TIMEOUT || !wait_gave_up()) *status = GIPB200_OK;
+  }
+  return GIPB200_OK;
+}
+
 static Stream64 stream64(const Pcg& P) {
   const Packed64& o = P.op64;
   return {o.delta.p, o.bits == 4 ? (const void*)o.idx4.p : (const void*)o.idx8.p, o.base.p,
@@ -815,8 +855,8 @@ static Stream64 stream64(const Pcg& P) {
 
 int Pcg::enqueue_one_launch(const double* b, double* x, const double* x0, cudaStream_t s) {
   if (one.form == OneLaunch::kSolve) return enqueue_solve_launch(b, x, x0, s);
-  Args64 A{L->view(), b, x0, dinv.p, x, one.pair.p, one.slots.p, sc.p, prm.tol, n, n_all,
-           prm.mode, prm.maxit};
+  Args64 A{L->view(), b,     x0,    dinv.p,   x,        one.pair.p, one.slots.p, sc.p,
+           gave_up,   prm.tol, n, n_all, prm.mode, prm.maxit};
   launches += 1;
   if (one.form != OneLaunch::kBlock && one.form != OneLaunch::kCluster)
     GIPB_CUDA(cudaMemsetAsync(one.slots.p, 0, one.slots.n * sizeof(ulonglong2), s));

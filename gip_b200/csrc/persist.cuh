@@ -8,8 +8,8 @@
 
 namespace gipb200 {
 
-// A grid wait that would never end gives up after about 2 s of SM clock.
-constexpr long long kGridSpinCycles = 4000000000LL;
+// A grid wait that would never end gives up after about 2 s of SM clock (a check of that: 20 ms).
+constexpr long long kGridSpinCycles = 4000000000LL, kCheckSpinCycles = 40000000LL;
 constexpr int kGridSums = 5;       // sums per grid reduction
 constexpr int kGridCtasMax = 256;  // CTAs of a grid reduction (each polled by one thread)
 // 16-byte slots of one grid's reductions: [2 parities][kGridSums][CTA], then the arrival
@@ -50,15 +50,23 @@ struct GridScope {
   unsigned* count;
   unsigned epoch;
   int ncta, rank;
+  long long spin;  // cycles after which a wait gives up
   bool ok;  // false: a wait gave up (the same in every thread after the call that noticed)
 };
 
-__device__ __forceinline__ GridScope grid_begin(ulonglong2* slots, int rank, int ncta) {
+__device__ __forceinline__ GridScope grid_begin(ulonglong2* slots, int rank, int ncta,
+                                                 long long spin = kGridSpinCycles) {
   return GridScope{slots, reinterpret_cast<unsigned*>(slots + (size_t)2 * kGridSums * ncta), 0u,
-                   ncta, rank, true};
+                   ncta, rank, spin, true};
 }
 __device__ __forceinline__ GridScope grid_begin(ulonglong2* slots) {
   return grid_begin(slots, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// A solve one of whose waits gave up tells the host, whoever enqueued it (pinned memory).
+__device__ __forceinline__ void report_gave_up(int* flag) {
+  *static_cast<volatile int*>(flag) = 1;
+  __threadfence_system();
 }
 
 // FENCE: the reduction is also a barrier for global memory (what any thread of the grid wrote
@@ -94,7 +102,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[W], GridScope& G) {
       while (true) {
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(G.count) : "memory");
         if ((int)(c - target) >= 0) break;
-        if (clock64() - t0 > kGridSpinCycles) {
+        if (clock64() - t0 > G.spin) {
           s_fail = 1;
           break;
         }
@@ -116,7 +124,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[W], GridScope& G) {
         while (true) {
           slot_load(set + (size_t)k * G.ncta + threadIdx.x, t[k], e);
           if (e == G.epoch) break;
-          if (clock64() - t0 > kGridSpinCycles) {
+          if (clock64() - t0 > G.spin) {
             s_fail = 1;
             break;
           }
@@ -160,7 +168,7 @@ __device__ __forceinline__ bool grid_wait(GridScope& G) {
     while (true) {
       asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(G.count) : "memory");
       if ((int)(c - target) >= 0) break;
-      if (clock64() - t0 > kGridSpinCycles) {
+      if (clock64() - t0 > G.spin) {
         s_fail = 1;
         break;
       }

@@ -181,6 +181,7 @@ struct SolveArgs {
   double* rpart;
   int vblocks;              // blocks of the kernel whose order the sum keeps
   PcgScalars* S;
+  int* gave_up;             // host flag: a wait gave up
   ulonglong2* slots;
   const CycleOp<T>* ops;    // null: no preconditioner beyond the Jacobi scaling
   int nops;                 // level 0's residual first, its smoothing after the last
@@ -932,6 +933,7 @@ __device__ __forceinline__ void mixed_solve(const SolveArgs<float>& A, Team& g) 
     }
     ok = precondition();
   }
+  if (!ok && lead) report_gave_up(A.gave_up);
   if (g.rank() == 0 && lead) {
     PcgScalars* S = A.S;
     S->rz = T.rz;
@@ -973,6 +975,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed_cluster(const __grid_cons
   ClusterTeam g = cluster_team(red);
   mixed_solve<AMG>(A, g);
   cluster_barrier();  // no CTA leaves while another may still write its sums
+}
+
+// One CTA of a group that claims two: a solve without rows, whose first sum waits for a CTA that
+// does not exist, or a barrier of that group.
+__global__ void __launch_bounds__(kThreads, 1) k_mixed_wait_check(const __grid_constant__ SolveArgs<float> A,
+                                                                  int barrier_only) {
+  GridTeam g{grid_begin(A.slots, 0, 2, kCheckSpinCycles)};
+  if (!barrier_only) {
+    mixed_solve<false>(A, g);
+  } else if (!barrier(g) && threadIdx.x == 0) {
+    report_gave_up(A.gave_up);
+    A.S->status = GIPB200_ERR_TIMEOUT;
+  }
 }
 
 // The solves of a batch in one launch, a group of CTAs per instance; groups never wait on one
@@ -1131,6 +1146,7 @@ __device__ __forceinline__ void tol_amg_solve(const SolveArgs<double>& A, Team& 
     }
     __syncthreads();
   }
+  if (!ok && lead) report_gave_up(A.gave_up);
   if (g.rank() == 0 && lead) {
     PcgScalars* S = A.S;
     S->rz = T.rz;
@@ -1386,6 +1402,7 @@ SolveArgs<float> mixed_args(Pcg& P, const double* b, const double* bp, double* x
   A.rpart = P.one.rd.p + P.n;
   A.vblocks = P.blocks_spmv;
   A.S = P.sc.p;
+  A.gave_up = P.gave_up;
   A.slots = P.one.slots.p;
   A.ops = reinterpret_cast<const CycleOp<float>*>(P.one.ops.p);
   A.nops = P.one.nops;
@@ -1403,6 +1420,16 @@ SolveArgs<float> mixed_args(Pcg& P, const double* b, const double* bp, double* x
   return A;
 }
 }  // namespace
+
+void Pcg::launch_wait_check(bool barrier_only, ulonglong2* slots, cudaStream_t s) {
+  SolveArgs<float> A{};
+  A.pin_row = -1;
+  A.S = sc.p;
+  A.gave_up = gave_up;
+  A.slots = slots;
+  A.maxit = A.max_outer = 1;
+  k_mixed_wait_check<<<1, kThreads, 0, s>>>(A, barrier_only ? 1 : 0);
+}
 
 int Pcg::enqueue_solve_launch(const double* b, double* x, const double* x0, cudaStream_t s) {
   if (!one.cluster)
@@ -1430,6 +1457,7 @@ int Pcg::enqueue_solve_launch(const double* b, double* x, const double* x0, cuda
   A.r = r.p;
   A.q = Ap.p;
   A.S = sc.p;
+  A.gave_up = gave_up;
   A.slots = one.slots.p;
   A.ops = reinterpret_cast<const CycleOp<double>*>(one.ops.p);
   A.nops = one.nops;

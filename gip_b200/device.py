@@ -350,6 +350,8 @@ class DnsEngine:
         L.call("gipb200_dns_history", self.handle, C.byref(steps), _hptr(out["time"]),
                _hptr(out["dt"]), _hptr(out["massr"]), _hptr(out["iters"]), _hptr(out["rr"]),
                _hptr(out["outer"]), _hptr(out["kernels"]))
+        out["status"] = np.zeros(n, np.int32)  # of the pressure solves
+        L.call("gipb200_dns_solve_status", self.handle, n, _hptr(out["status"]), None)
         return out
 
     PHASES = ("predictor", "poisson_rhs", "pcg", "ghost_copy", "correction", "mass_fluxes",
@@ -530,7 +532,7 @@ class DnsBatch:
         return g.value, n
 
     def solver_status(self, stream=None) -> int:
-        """Nonzero when a barrier of the persistent solve gave up since the last call."""
+        """Nonzero when a wait of a one-launch solve gave up since the last call."""
         e = C.c_int()
         L.call("gipb200_batch_solver_status", self.handle, _stream(stream), C.byref(e))
         return e.value

@@ -180,7 +180,7 @@ enum { GIPB200_PRECOND_JACOBI = 0, GIPB200_PRECOND_AMG = 1 };
 typedef struct {
   int iterations;        /* FIXED/TOL: PCG iterations; MIXED: inner iterations summed */
   int outer;             /* MIXED: FP64 residual replacements                         */
-  int status;            /* GIPB200_OK / BREAKDOWN / NOT_CONVERGED                    */
+  int status;            /* GIPB200_OK / BREAKDOWN / NOT_CONVERGED / TIMEOUT          */
   double rr;             /* r.r at exit (MIXED: true FP64 residual)                   */
   double bb;             /* b.b                                                       */
 } gipb200_pcg_result;
@@ -340,6 +340,17 @@ int gipb200_dns_advance(gipb200_dns E, int nsteps, void* stream);
 int gipb200_dns_history(gipb200_dns E, int* steps_taken, double* h_time, double* h_dt,
                         double* h_massr, int* h_iters, double* h_rr, int* h_outer,
                         int* h_kernels);
+/* The pressure solves' statuses (GIPB200_OK, NOT_CONVERGED, BREAKDOWN, TIMEOUT) of the first
+ * min(steps taken, max_steps) steps; *steps_out (may be NULL) = steps written.  Synchronises
+ * the device.  After a TIMEOUT (a device wait of a solve that runs as one launch gave up, after
+ * about 2 s) the engine's state is not valid and further steps are refused with
+ * GIPB200_ERR_TIMEOUT until a snapshot is restored. */
+int gipb200_dns_solve_status(gipb200_dns E, int max_steps, int* h_status, int* steps_out);
+/* Runs one-launch solves and a barrier that wait for a thread block that does not exist, on the
+ * engine's solver: *h_status = GIPB200_ERR_TIMEOUT when each gave up (after about 20 ms here)
+ * and recorded it, as designed; the engine then refuses steps as after a timeout of its own.
+ * The context stays usable.  Synchronises `stream`. */
+int gipb200_dns_check_bounded_wait(gipb200_dns E, void* stream, int* h_status);
 /* Per-phase timing report (what a GIP_TimerB200 channel per phase would give): advances
  * one timestep with host-driven loops (no graph) and CUDA events on `stream` between
  * GIP_DNS's phases, and writes their durations in ms to h_ms[7]: predictor (Ec, D/C
@@ -473,8 +484,9 @@ int gipb200_batch_balance(gipb200_batch B, const double* weights);
 /* The persistent solve's grid and each instance's CTAs (h_ncta: one per instance, or
  * null); 0 when the batch solves inside its branches. */
 int gipb200_batch_layout(gipb200_batch B, int* grid, int* h_ncta);
-/* *h_err = nonzero when a group barrier of the persistent solve gave up waiting (about 2 s)
- * since the last call, which clears it; the instances' results are then not valid.
+/* *h_err = nonzero when a wait of the persistent solve, or of an instance's solve that runs as
+ * one launch, gave up (after about 2 s) since the last call, which clears it; the instances'
+ * results are then not valid.
  * Synchronises `stream`. */
 int gipb200_batch_solver_status(gipb200_batch B, void* stream, int* h_err);
 /* Runs one persistent-solve launch whose group barrier waits for a CTA that does not exist:
