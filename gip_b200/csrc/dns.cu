@@ -1576,13 +1576,17 @@ int gipb200_dns_snapshot(gipb200_dns Dh, int restore, void* stream) {
   constexpr int ns = (int)(sizeof(state) / sizeof(state[0]));
   static_assert(ns < StateCopy::kMost && sizeof(DnsScalars) % 8 == 0, "the copy's segments");
   if (!restore) {
-    if (E.snap.empty()) {
-      for (int k = 0; k < ns; ++k) {
-        DevBuf<double>* b = new DevBuf<double>();
-        E.snap.push_back(b);
-        GIPB_TRY(b->alloc(state[k]->n));
+    if (E.snap.empty()) {  // all of its buffers or none: the copy below writes every one
+      int st = E.snap_sc.alloc(1);
+      for (int k = 0; k < ns && st == GIPB200_OK; ++k) {
+        E.snap.push_back(new DevBuf<double>());
+        st = E.snap.back()->alloc(state[k]->n);
       }
-      GIPB_TRY(E.snap_sc.alloc(1));
+      if (st != GIPB200_OK) {
+        for (auto* b : E.snap) delete b;
+        E.snap.clear();
+        return st;
+      }
     }
   } else if (E.snap.empty() || E.snap_steps < 0) {
     return fail(GIPB200_ERR_STATE, "no snapshot taken");

@@ -69,6 +69,7 @@ struct DevBuf {
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T));
     if (e != cudaSuccess) {
       p = nullptr;
+      (void)cudaGetLastError();  // the status says it; a later launch check must not find it
       return fail(GIPB200_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", count * sizeof(T),
                   cudaGetErrorString(e));
     }
