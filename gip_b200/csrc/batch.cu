@@ -98,7 +98,11 @@ int Batch::plan_groups() {
 int Batch::capture() {
   for (auto d : inst) d->E.graph_kernels = 0;
   groups.on = false;
-  if (!persistent) GIPB_TRY(plan_groups());
+  if (!persistent) {
+    const int st = plan_groups();
+    if (st != GIPB200_OK) groups.release();
+    if (st != GIPB200_OK && st != GIPB200_ERR_NOMEM) return st;  // no memory: in the branches
+  }
   GIPB_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
   int st = GIPB200_OK;
   int rc = [&]() -> int {

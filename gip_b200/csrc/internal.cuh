@@ -239,6 +239,15 @@ struct Packed64 {
   DevBuf<int> base;              // per slice, 8 slots
   DevBuf<unsigned char> plain;   // per slice
   DevBuf<double> table;          // 16 or 256 entries
+  void release() {
+    bits = 0;
+    delta.release();
+    idx4.release();
+    idx8.release();
+    base.release();
+    plain.release();
+    table.release();
+  }
 };
 int pack64(const Sell& S, int cols, bool keep_zeros, Packed64* out, cudaStream_t s);
 int launch_packed_spmv(const Sell& A, const Packed64& P, const double* x, double* y, double alpha,

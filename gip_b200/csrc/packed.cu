@@ -4,18 +4,20 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 
 #include "device.cuh"
 #include "internal.cuh"
 
 namespace gipb200 {
 
+namespace {
+
 // cols: columns below it are kept; entries of later ones (ghost cells whose stored values the
 // caller knows to be zeros) become padding.  keep_zeros: a stored zero is an entry with a
 // table value of its own (its product with an infinity is a NaN, as in the sliced layout);
 // else it is padding that gathers its column and multiplies by table entry 0.
-int pack64(const Sell& S, int cols, bool keep_zeros, Packed64* out, cudaStream_t s) {
-  out->bits = 0;
+int build(const Sell& S, int cols, bool keep_zeros, Packed64* out, cudaStream_t s) {
   const int ns = S.nslices;
   const long long nslots = S.nslots;
   if (ns == 0 || nslots == 0) return GIPB200_OK;
@@ -101,6 +103,22 @@ int pack64(const Sell& S, int cols, bool keep_zeros, Packed64* out, cudaStream_t
   out->bits = nib;
   out->slots = longest <= 7 ? 7 : 8;
   return GIPB200_OK;
+}
+
+}  // namespace
+
+// The packed copy is a second one: where there is no memory for it the operator is used without.
+int pack64(const Sell& S, int cols, bool keep_zeros, Packed64* out, cudaStream_t s) {
+  out->release();
+  int st;
+  try {
+    st = build(S, cols, keep_zeros, out, s);
+  } catch (const std::bad_alloc&) {
+    st = GIPB200_ERR_NOMEM;
+  }
+  if (st == GIPB200_OK) return GIPB200_OK;
+  out->release();
+  return st == GIPB200_ERR_NOMEM ? GIPB200_OK : st;
 }
 
 namespace {

@@ -72,6 +72,13 @@ struct OneLaunch {
   DevBuf<double> rd;             // kSolve, mixed: the FP64 residual and partial sums of it
   bool cluster = false;          // kSolve: over a cluster instead of a cooperative grid
   DevBuf<ulonglong2> slots;      // grid reductions
+  void release() {
+    form = kNone;
+    pair.release();
+    ops.release();
+    rd.release();
+    slots.release();
+  }
 };
 
 struct Pcg {
@@ -203,6 +210,7 @@ struct Pcg {
   int build_packed64(cudaStream_t s);
   void follow_values();
   int plan_one_launch(cudaStream_t s);
+  int choose_one_launch(cudaStream_t s);
   int plan_solve_launch(cudaStream_t s);
   int enqueue_solve_launch(const double* b, double* x, const double* x0, cudaStream_t s);
   void launch_wait_check(bool barrier_only, ulonglong2* slots, cudaStream_t s);
@@ -231,6 +239,12 @@ struct SolveGroups {
   DevBuf<unsigned char> items;   // the solves' arguments
   DevBuf<int> owner;             // solver of every CTA
   DevBuf<ulonglong2> slots;      // the groups' barriers
+  void release() {
+    on = false;
+    items.release();
+    owner.release();
+    slots.release();
+  }
   int plan(const std::vector<Pcg*>& solvers, const std::vector<const double*>& b,
            const std::vector<double*>& x, const std::vector<const double*>& x0, cudaStream_t s);
   int launch(cudaStream_t s) const;

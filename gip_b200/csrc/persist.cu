@@ -29,6 +29,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "persist.cuh"
@@ -739,10 +740,23 @@ int Pcg::solve_form() {
   }
 }
 
-// Which one-launch form runs this solver's solves.
+// A solver that found no memory for its one-launch form solves kernel by kernel.
 int Pcg::plan_one_launch(cudaStream_t s) {
-  one.form = OneLaunch::kNone;
+  one.release();
   planned_version = L->version;
+  int st;
+  try {
+    st = choose_one_launch(s);
+  } catch (const std::bad_alloc&) {
+    st = GIPB200_ERR_NOMEM;
+  }
+  if (st == GIPB200_OK) return GIPB200_OK;
+  one.release();
+  return st == GIPB200_ERR_NOMEM ? GIPB200_OK : st;
+}
+
+// Which one-launch form runs this solver's solves.
+int Pcg::choose_one_launch(cudaStream_t s) {
   if (prm.mode == GIPB200_PCG_MIXED || prm.precond != GIPB200_PRECOND_JACOBI)
     return plan_solve_launch(s);
   if (n <= 0 || !L->rows_nonempty || getenv("GIPB200_NO_ONE_LAUNCH")) return GIPB200_OK;

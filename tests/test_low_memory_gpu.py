@@ -52,3 +52,71 @@ def test_snapshot_that_found_no_memory_can_be_taken_later(gpu, left_mb):
     for k in kept:
         assert np.array_equal(E.field(k), later[k]), k
         assert not np.array_equal(kept[k], later[k]), k
+
+
+def _created(make):
+    try:
+        return make()
+    except _lib.GipB200Error as e:
+        assert e.status == _lib.ERR_NOMEM or "out of memory" in str(e), e
+        return None
+
+
+def test_large_handles_need_no_memory_for_the_packed_copy(gpu, monkeypatch):
+    # whatever memory the sliced layout fits in is enough for a handle: the packed copy is left
+    # out where it does not fit beside it; the products are the same bits
+    from gip_b200.device import DeviceMatrix
+    from test_one_launch_gpu import _band
+    n = 200000
+    m = _band(n, n, seed=2)
+    x = torch.randn(n, dtype=torch.float64, device="cuda")
+    want = DeviceMatrix(m).spmv(x, torch.zeros_like(x)).cpu()
+    y = torch.zeros_like(x)
+    fits = []
+    for left_mb in range(10, 60, 2):
+        with memory_left(left_mb << 20):
+            monkeypatch.setenv("GIPB200_NO_PACK", "1")
+            plain = _created(lambda: DeviceMatrix(m))
+            fits.append(plain is not None)
+            if plain is not None:
+                plain.close()
+                monkeypatch.delenv("GIPB200_NO_PACK")
+                A = _created(lambda: DeviceMatrix(m))
+                assert A is not None, left_mb
+                y.zero_()
+                assert torch.equal(A.spmv(x, y).cpu(), want)
+                A.close()
+    assert True in fits and False in fits  # the range crosses what the handle needs
+
+
+SOLVERS = [("stream", 1500000, dict(mode="fixed", maxit=5), range(32, 120, 4)),
+           ("mixed", 1500000, dict(mode="mixed", maxit=500, tol=1e-8, inner_tol=0.1, max_outer=50),
+            range(64, 320, 16)),
+           ("tol_amg", 150000, dict(mode="tol", maxit=100, tol=1e-8, precond="amg"),
+            range(16, 96, 6))]
+
+
+@pytest.mark.parametrize("name,n,kw,left", SOLVERS, ids=[s[0] for s in SOLVERS])
+def test_solvers_need_no_memory_for_one_launch(gpu, monkeypatch, name, n, kw, left):
+    # where the kernel-by-kernel solver fits, the solver can be created and solves
+    from gip_b200.device import DeviceMatrix, PcgSolver
+    from test_one_launch_gpu import _band
+    A = DeviceMatrix(_band(n, n, seed=2))
+    b = torch.randn(n, dtype=torch.float64, device="cuda")
+    x, x0 = torch.zeros_like(b), torch.zeros_like(b)
+    fits, forms = [], set()
+    for left_mb in left:
+        with memory_left(left_mb << 20):
+            monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+            K = _created(lambda: PcgSolver(A, **kw))
+            fits.append(K is not None)
+            if K is not None:
+                K.close()
+                monkeypatch.delenv("GIPB200_NO_ONE_LAUNCH")
+                S = _created(lambda: PcgSolver(A, **kw))
+                assert S is not None, left_mb
+                forms.add(S.solve_form())
+                assert S.solve(b, x, x0)["status"] == 0
+                S.close()
+    assert True in fits and False in fits, fits  # the range crosses what the solver needs
+    assert len(forms - {"loop"}) == 1, forms
