@@ -299,6 +299,8 @@ def host_loop_pcg(A: DeviceMatrix, Dg: DeviceMatrix, dinv: torch.Tensor, b: torc
                                    ("matrix_spmv_dot", "cg_update_dot", "cg_direction"))
     pAp = C.c_void_p(sc.data_ptr() + 8)
     dp, dAx, dx, dr, dz, dd, dsc = (_dptr(t) for t in (p, Ax, x, r, z, dinv, sc))
+    if maxit > 0:
+        A._check(p, n, Ax)  # what every spmv_dot of the loop is called with
     for _ in range(maxit):
         st = spmv_dot(A.handle, dp, dAx, n, pAp, s) or \
             update(A.handle, n, dx, dr, dz, dp, dAx, dd, dsc, s) or direction(n, dp, dz, dsc, s)
