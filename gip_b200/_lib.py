@@ -120,6 +120,8 @@ _SIGNATURES = {
     "gipb200_pcg_destroy": (_I, [_VP]),
     "gipb200_pcg_get_info": (_I, [_VP, C.POINTER(PcgInfo)]),
     "gipb200_check_bounded_wait": (_I, [_VP, C.POINTER(_I)]),
+    "gipb200_pcg_share_gpu": (_I, [_VP, _I]),
+    "gipb200_dns_share_gpu": (_I, [_VP, _I]),
     "gipb200_pcg_solve_form": (_I, [_VP, C.POINTER(_I)]),
     "gipb200_pcg_kernel_time": (_I, [_VP, _I, _VP, C.POINTER(_D), C.POINTER(_D)]),
     "gipb200_pcg_solve": (_I, [_VP, _VP, _VP, _VP, _VP, C.POINTER(PcgResult)]),

@@ -1544,6 +1544,16 @@ int gipb200_dns_set_launch(gipb200_dns Dh, int spmv_blocks, int vec_blocks) {
   return GIPB200_OK;
 }
 
+int gipb200_dns_share_gpu(gipb200_dns Dh, int on) {
+  if (!Dh) return fail(GIPB200_ERR_ARG, "null engine");
+  Dns& E = Dh->E;
+  if (E.pcg.shared_gpu != (on != 0)) {
+    E.pcg.shared_gpu = on != 0;
+    E.drop_graph();  // the next step captures the other form of the solve
+  }
+  return GIPB200_OK;
+}
+
 int gipb200_dns_get_info(gipb200_dns Dh, gipb200_dns_info* info) {
   if (!Dh || !info) return fail(GIPB200_ERR_ARG, "null argument");
   const Dns& E = Dh->E;

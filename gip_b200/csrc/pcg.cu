@@ -1883,6 +1883,12 @@ int gipb200_pcg_get_info(gipb200_pcg S, gipb200_pcg_info* info) {
   return GIPB200_OK;
 }
 
+int gipb200_pcg_share_gpu(gipb200_pcg S, int on) {
+  if (!S) return fail(GIPB200_ERR_ARG, "null solver");
+  S->P.shared_gpu = on != 0;
+  return GIPB200_OK;
+}
+
 int gipb200_pcg_solve_form(gipb200_pcg S, int* form) {
   if (!S || !form) return fail(GIPB200_ERR_ARG, "null argument");
   *form = S->P.solve_form();

@@ -149,9 +149,15 @@ struct Pcg {
   Packed64 op64;                 // L packed (bits = 0: not)
   unsigned planned_version = 0;  // of L's values, when op64 and `one` were made from them
   OneLaunch one;
-  // several solvers advance side by side on one GPU (a batch): forms that claim every SM at
-  // once (the cooperative ones) would take turns, so only the cluster form runs
-  bool shared_gpu = false;
+  // Other work runs beside this solver's on the GPU: forms that claim every SM (the cooperative
+  // ones) would take turns with it, so only those over one block or cluster run.  Eight 44^3 mixed
+  // AMG engines on eight streams take 46.5 ms for ten steps in cooperative launches and 13.7
+  // shared, one alone 6.0 and 8.7; two 48^3 fixed ones 12.3 / 19.9, eight 49.7 / 32.5.  Nothing
+  // here decides it: the rounding of the dots, which differs from form to form, would then
+  // depend on what else the program runs.  shared_gpu: on
+  // request (gipb200_dns_share_gpu, gipb200_pcg_share_gpu).  in_batch: an instance in a batch's
+  // branches; its preconditioned solves stay kernels there.
+  bool shared_gpu = false, in_batch = false;
   // a step history counts the kernels of every solve against its iterations: the mixed form
   // with Jacobi and the FP64 form with AMG of an engine keep their kernels
   bool counted = false;
@@ -159,8 +165,9 @@ struct Pcg {
     if (one.form == OneLaunch::kSolve && counted &&
         (prm.mode == GIPB200_PCG_MIXED) != (prm.precond == GIPB200_PRECOND_AMG))
       return false;
-    return one.form == OneLaunch::kBlock || one.form == OneLaunch::kCluster ||
-           (one.form != OneLaunch::kNone && !shared_gpu);
+    if (one.form == OneLaunch::kBlock || one.form == OneLaunch::kCluster) return true;
+    if (one.form == OneLaunch::kNone || in_batch) return false;
+    return !shared_gpu || (one.form == OneLaunch::kSolve && one.cluster);
   }
   int solve_form();  // GIPB200_SOLVE_* of the next solve
   // scalars and reduction scratch

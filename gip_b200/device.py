@@ -239,6 +239,10 @@ class PcgSolver:
                C.byref(nb))
         return ms.value, nb.value
 
+    def share_gpu(self, on: bool = True) -> None:
+        """Other work runs on the GPU beside this solver's: no solve claims every SM."""
+        L.call("gipb200_pcg_share_gpu", self.handle, int(bool(on)))
+
     def solve_form(self) -> str:
         """How the next solve runs: "loop" (kernel by kernel) or its one-launch form."""
         f = C.c_int()
@@ -455,6 +459,11 @@ class DnsEngine:
     def snapshot(self, restore: bool = False, stream=None) -> None:
         """Save (or restore) the whole timestep state on the device."""
         L.call("gipb200_dns_snapshot", self.handle, int(restore), _stream(stream))
+
+    def share_gpu(self, on: bool = True) -> None:
+        """For engines that advance side by side on several streams: no pressure solve claims
+        every SM, so their steps overlap."""
+        L.call("gipb200_dns_share_gpu", self.handle, int(bool(on)))
 
     def set_launch(self, spmv_blocks: int = 0, vec_blocks: int = 0) -> None:
         L.call("gipb200_dns_set_launch", self.handle, spmv_blocks, vec_blocks)

@@ -223,6 +223,11 @@ enum {
   GIPB200_SOLVE_PRECOND_GRID = 6     /* MIXED, or TOL with AMG: cooperative grid          */
 };
 int gipb200_pcg_solve_form(gipb200_pcg S, int* form);
+/* No counterpart in the reference: on != 0 says that other work runs on the GPU beside this
+ * solver's (solves of other host threads, steps on other streams).  Solves that would claim
+ * every SM for their whole duration (GRID, STREAM, PRECOND_GRID), and so take turns, run kernel
+ * by kernel instead.  Off by default: a solve alone on the GPU is faster in one launch. */
+int gipb200_pcg_share_gpu(gipb200_pcg S, int on);
 /* No counterpart in the reference: times `reps` launches of the solver's SpMV-dot kernel
  * (FP64 forms: the FP64 kernel; MIXED: the FP32 kernel of its operator layout) on its
  * current search direction, with CUDA events on `stream`; returns the mean launch time and
@@ -417,6 +422,11 @@ int gipb200_dns_snapshot(gipb200_dns E, int restore, void* stream);
  * dot-product partial sums (results stay deterministic for a given shape).  The next
  * step re-captures its graph. */
 int gipb200_dns_set_launch(gipb200_dns E, int spmv_blocks, int vec_blocks);
+
+/* gipb200_pcg_share_gpu for the engine's pressure solver: on != 0 for engines that advance side
+ * by side on several streams, whose steps then overlap.  The next step re-captures its graph.
+ * (The instances of a batch need no such call.) */
+int gipb200_dns_share_gpu(gipb200_dns E, int on);
 
 /* Algorithmic bytes of each phase of one timestep, in the order of
  * gipb200_dns_step_phases (h_bytes[7]; stored operator values and indices once, gathered
