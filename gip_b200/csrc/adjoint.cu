@@ -397,8 +397,8 @@ int gipb200_adjoint_create(const gipb200_dns_ops* ops, const double* h_u0, const
     dp.pcg.precond = prm->precond;
     dp.use_graph = 1;
     dp.reorder = 0;
+    A.E.count_kernels = false;  // no history of kernels is read from an adjoint's engine
     GIPB_TRY(dns_init(A.E, ops, h_u0, h_v0, h_w0, h_dxs, &dp));
-    A.E.pcg.counted = false;  // no history of kernels is read from an adjoint's engine
     A.u0.assign(h_u0, h_u0 + NO);
     A.v0.assign(h_v0, h_v0 + NO);
     A.w0.assign(h_w0, h_w0 + NO);

@@ -242,7 +242,7 @@ int gipb200_batch_create(int n, const gipb200_dns_ops* const* ops, const double*
       gipb200_dns d = nullptr;
       GIPB_TRY(gipb200_dns_create(ops[i], h_u[i], h_v[i], h_w[i], h_dxs[i], &params[i], &d));
       B.inst.push_back(d);
-      d->E.pcg.in_batch = true;
+      d->E.pcg.join_batch();
       cudaStream_t s;
       GIPB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
       B.streams.push_back(s);

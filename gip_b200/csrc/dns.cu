@@ -1241,7 +1241,7 @@ int dns_init(Dns& E, const gipb200_dns_ops* ops, const double* h_u, const double
     trace("merged faces, fields");
     E.setup_s[1] = since(t_ops);  // device layouts of the operators, fields
     const auto t_pcg = std::chrono::steady_clock::now();
-    E.pcg.counted = true;
+    E.pcg.counted = E.count_kernels;
     GIPB_TRY(E.pcg.init(&E.L, NO, prm->pcg, 0));
     trace("pressure solver");
     E.setup_s[2] = since(t_pcg);  // the pressure solver (FP32 operator, packing, AMG)

@@ -77,6 +77,7 @@ struct Dns {
   DevBuf<double> partials;
   DevBuf<unsigned> ticket;
   ReduceScratch rs{};
+  bool count_kernels = true;     // the history's kernels are read (set before dns_init)
   int steps_enqueued = 0;
   bool started = false;
   cudaStream_t cap_stream = nullptr;

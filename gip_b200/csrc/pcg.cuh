@@ -158,17 +158,16 @@ struct Pcg {
   // request (gipb200_dns_share_gpu, gipb200_pcg_share_gpu).  in_batch: an instance in a batch's
   // branches; its preconditioned solves stay kernels there.
   bool shared_gpu = false, in_batch = false;
-  // a step history counts the kernels of every solve against its iterations: the mixed form
-  // with Jacobi and the FP64 form with AMG of an engine keep their kernels
+  // A step history counts the kernels of every solve against its iterations: the mixed form
+  // with Jacobi and the FP64 form with AMG of an engine keep their kernels, and plan nothing else
+  // (set before init).
   bool counted = false;
   bool one_launch() const {
-    if (one.form == OneLaunch::kSolve && counted &&
-        (prm.mode == GIPB200_PCG_MIXED) != (prm.precond == GIPB200_PRECOND_AMG))
-      return false;
     if (one.form == OneLaunch::kBlock || one.form == OneLaunch::kCluster) return true;
     if (one.form == OneLaunch::kNone || in_batch) return false;
     return !shared_gpu || (one.form == OneLaunch::kSolve && one.cluster);
   }
+  void join_batch();  // in_batch, and the buffers of forms that then never run given back
   int solve_form();  // GIPB200_SOLVE_* of the next solve
   // scalars and reduction scratch
   DevBuf<PcgScalars> sc;

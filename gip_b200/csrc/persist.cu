@@ -728,6 +728,11 @@ int Pcg::ghosts_zero(cudaStream_t s, bool* zero) const {
   return GIPB200_OK;
 }
 
+void Pcg::join_batch() {
+  in_batch = true;
+  if (one.form == OneLaunch::kGrid || one.form == OneLaunch::kStream) one.release();
+}
+
 int Pcg::solve_form() {
   follow_values();
   if (!one_launch()) return GIPB200_SOLVE_LOOP;

@@ -1352,7 +1352,7 @@ int Pcg::plan_solve_launch(cudaStream_t s) {
   size_t bytes = 0;
   std::vector<unsigned char> raw;
   if (mixed) {
-    if (rec) return GIPB200_OK;
+    if (rec || (counted && !amg)) return GIPB200_OK;
     if (amg) {
       std::vector<CycleOp<float>> ops;
       if (!cycle_ops<float>(*amg, r32.p, warps, &ops)) return GIPB200_OK;
@@ -1370,6 +1370,7 @@ int Pcg::plan_solve_launch(cudaStream_t s) {
     GIPB_TRY(ghosts_zero(s, &zero));
     if (!zero) return GIPB200_OK;
     GIPB_TRY(build_packed64(s));
+    if (counted) return GIPB200_OK;  // the loop reads the packed operator too
     one.nops = (int)ops.size();
     bytes = ops.size() * sizeof(ops[0]);
     raw.assign((unsigned char*)ops.data(), (unsigned char*)ops.data() + bytes);

@@ -120,3 +120,24 @@ def test_solvers_need_no_memory_for_one_launch(gpu, monkeypatch, name, n, kw, le
                 S.close()
     assert True in fits and False in fits, fits  # the range crosses what the solver needs
     assert len(forms - {"loop"}) == 1, forms
+
+
+def test_engines_hold_no_buffers_of_forms_they_never_run(gpu, monkeypatch):
+    # an engine with mixed Jacobi keeps the kernel-by-kernel loop: it takes the memory of an engine
+    # that plans nothing else (at 100^3 the unused pairs and residual would be 16 MB; a difference
+    # of one 2 MB granule of the allocator is allowed)
+    from gip_b200.device import DnsEngine
+    case, _ = cavity.generate(100, re=100.0)
+    kw = dict(gamma=0.01, pcg_mode="mixed", maxit=500, tol=1e-6, inner_tol=0.3, max_outer=100)
+    DnsEngine(case, **kw).close()
+    used = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("GIPB200_NO_ONE_LAUNCH", "1")
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        E = DnsEngine(case, **kw)
+        torch.cuda.synchronize()
+        used.append(before - torch.cuda.mem_get_info()[0])
+        E.close()
+    assert abs(used[0] - used[1]) <= 2 << 20, used
