@@ -1274,9 +1274,18 @@ double Pcg::iteration_bytes() const {
     const double spmv = (cop.enabled ? cop.bytes_per_launch : plain + 16.0 * nn) +
                         (rec ? 4.0 * nn : 0.0);  // the previous A p read by the recurrence
     double b = spmv + 24.0 * nn;  // SpMV-dot (direction formed inside), y/r update
+    if (one_launch()) b += 8.0 * nn;  // (z, p) pairs: z passes the update too
     if (amg) b += amg->cycle_bytes(cop.enabled ? cop.bytes_per_launch - 16.0 * nn : plain);
     return b;
   }
+  if (one_launch()) switch (one.form) {
+      case OneLaunch::kBlock:    // the state stays in registers and shared memory
+      case OneLaunch::kCluster: return 0.0;
+      case OneLaunch::kGrid: return 32.0 * nn;  // the (z, p) pairs written and read
+      case OneLaunch::kStream:   // p twice, dinv; x and p read and written; r, A p on chip
+        return packed64_bytes() + 48.0 * nn;
+      default: break;
+    }
   const double spmv = (op64.bits ? packed64_bytes() : 12.0 * nnz) + 16.0 * nn;
   if (amg64) {  // update (x, r read and written; p, Ap read), cycle, p = z + beta p
     const double a0 = (double)L->nslots * 12.0 + (L->nslices + 1.0) * 8.0;

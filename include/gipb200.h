@@ -404,6 +404,7 @@ typedef struct {
   double amg_complexity;       /* AMG: operator nonzeros of all levels / of the finest    */
   double amg_setup_s;          /* AMG: host setup time                                   */
   double iteration_bytes;      /* algorithmic bytes of one PCG iteration (with V-cycle)   */
+                               /* in the form it runs: 0 where its state stays on chip     */
   double replacement_bytes;    /* MIXED: bytes of one FP64 residual replacement           */
   int packed_residual;         /* MIXED: FP64 residual from the packed columns (1) or L   */
   int value_tables;            /* phase kernels (of 4: D/C products, right-hand side,     */
