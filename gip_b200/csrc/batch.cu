@@ -73,8 +73,10 @@ int Batch::branches(cudaEvent_t from, int part, int* st) {
     if (*st != GIPB200_OK) return *st;
     if (part == 1 && !persistent && E.pcg.lpacked) {  // what the grouped solve starts from
       const double* bp = nullptr;
+      const long long solves = E.pcg.launches;
       *st = E.pcg.enqueue_ghost_rhs(E.rhs.p, E.p0.p, streams[i], &bp);
       if (*st != GIPB200_OK) return *st;
+      E.graph_kernels += E.pcg.launches - solves;
     }
     GIPB_CUDA(cudaEventRecord(joins[i], streams[i]));
     GIPB_CUDA(cudaStreamWaitEvent(cap, joins[i], 0));
