@@ -23,3 +23,5 @@ def test_start_shorter_than_the_operators_columns_is_refused(gpu):
     x0, x, b, dinv = torch.zeros(n, **f), torch.zeros(2, n, **f), torch.ones(n, **f), torch.full((n,), 0.25, **f)
     with pytest.raises(ValueError):
         dv.host_loop_pcg(A, D, dinv, b, x, x0, 3)
+    A.close()  # not left to the collector: the caught error's frames hold them
+    D.close()

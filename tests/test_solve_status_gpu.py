@@ -64,3 +64,5 @@ def test_wait_that_gives_up_is_reported(gpu):
     with pytest.raises(_lib.GipB200Error):
         B.advance(1)
     assert B.solver_status() != 0 and B.solver_status() == 0
+    B.close()  # not left to the collector: a caught error's frames hold them
+    E.close()
