@@ -144,7 +144,7 @@ enum { kSell = 0, kCsr, kDense };
 enum { kOpPlain = 0, kOpResid, kOpScaleAdd, kOpSmooth, kOpDiagAdd };
 template <typename T>
 struct CycleOp {
-  int form, mode, nrows, nslices;
+  int form, mode, nrows;
   int lanes;               // threads per row (a power of two)
   int units;               // passes of a warp: 32 / lanes rows each
   int half, scaled;        // values in FP16; the gathered vector scaled by xs
@@ -172,7 +172,6 @@ struct SolveArgs {
   const double* x0;
   double* x;
   const double* scale;
-  const double* dinv;       // FP64 mode
   typename Pair2<T>::type* pair;
   T* r;
   T* q;                     // A p
@@ -1220,7 +1219,6 @@ bool cycle_ops(const AmgT<T>& M, const T* r, int warps, std::vector<CycleOp<T>>*
     o.form = A.lanes > 0 ? kCsr : kSell;
     o.mode = mode;
     o.nrows = A.nrows;
-    o.nslices = A.nslices;
     o.lanes = A.lanes;
     if (A.lanes == 0) {  // threads per sliced row: what covers an average row in one pass,
                          // while the operator still fits the grid's warps in two passes
@@ -1329,8 +1327,10 @@ int Pcg::plan_solve_launch(cudaStream_t s) {
   //   mixed AMG    63^3 63 / 131, 75^3 73 / 150, 128^3 244 / 189 (dependent launches)
   //   FP64 AMG     33^3 35 / 94, 63^3 57 / 135, 128^3 275 / 368, 200^3 1004 / 1061
   //   mixed Jacobi 33^3 8 / 23, 75^3 11 / 28, 128^3 34 / 45, 160^3 73 / 66
-  // beyond them the 16 to 32 warps a resident CTA leaves per SM gather slower than the 64 of
-  // the separate kernels.
+  // The 16 warps of a resident CTA per SM gather slower than the 64 of the separate kernels, which
+  // is what large systems are bound by: mixed AMG crosses between 75^3 and 128^3 and mixed Jacobi
+  // between 128^3 and 160^3, sizes between them not measured; FP64 AMG is 5% ahead at 200^3 still,
+  // and shares mixed Jacobi's line.
   const int most = mixed && with_amg ? 700000 : 2500000;
   if (n <= 0 || n > most || !L->rows_nonempty || getenv("GIPB200_NO_ONE_LAUNCH")) return GIPB200_OK;
   DeviceInfo di;
