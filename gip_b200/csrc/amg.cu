@@ -1489,8 +1489,7 @@ int AmgT<T>::enqueue(SellView<T> A0, const T* r, T* z0, PcgScalars* S, ReduceScr
   auto a_bytes = [&](int l) { return l == 0 ? a0_stream_bytes : stream_bytes(lv[l]->A); };
   // downward: pre-smooth from zero, residual, restriction (levels below the coarse tail)
   const bool u0 = unit0;  // level 0 never forms x0 = omega0 r
-  // a traced cycle runs kernel by kernel: its products are timed one by one
-  const bool small = tail_from < 0 && small_from > 0 && !tr;
+  const bool small = tail_from < 0 && small_from > 0;
   const int tf = small ? small_from : tail_from;
   for (int l = 0; l < L - 1 && (tf < 0 || l < tf); ++l) {
     const AmgLevel<T>& V = *lv[l];
@@ -1527,6 +1526,7 @@ int AmgT<T>::enqueue(SellView<T> A0, const T* r, T* z0, PcgScalars* S, ReduceScr
   }
   const AmgLevel<T>& C = *lv[L - 1];
   if (small) {  // the small levels and the coarsest, one launch of one cluster
+    GIPB_TRY(mark(tf, GIPB200_CYCLE_SMALL, small_bytes, GIPB200_FORM_SMALL));
     GIPB_TRY(launch_small_levels(*this, S, s));
   } else if (tf >= 0) {  // the small levels and the coarsest in one cooperative launch
     GIPB_TRY(mark(tf, GIPB200_CYCLE_TAIL, tail_bytes, GIPB200_FORM_TAIL));

@@ -139,6 +139,7 @@ struct AmgT {
   // Small levels (small_from.. and the dense coarsest solve) in one launch of one cluster
   // (persist_amg.cu); small_from < 0: one kernel per product.
   int small_from = -1, small_nops = 0, small_ctas = 0;
+  double small_bytes = 0.0;
   DevBuf<unsigned char> small_ops;
 
   // Hierarchy of the n x n operator (host CSR, FP64 values; columns < n), near-null

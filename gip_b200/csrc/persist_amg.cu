@@ -1500,6 +1500,14 @@ int plan_small_levels(AmgT<T>& M, cudaStream_t s) {
   if (st == GIPB200_ERR_NOMEM) return GIPB200_OK;  // without this launch, a kernel per product
   GIPB_TRY(st);
   GIPB_CUDA(cudaStreamSynchronize(s));
+  const double w = sizeof(T), nc = M.nc;
+  M.small_bytes = (nc * nc + 2.0 * nc) * w;
+  for (int l = t; l < L - 1; ++l) {  // residual, restriction, prolongation, smoothing
+    const AmgLevel<T>& V = *M.lv[l];
+    const double n = V.n, nn = M.lv[l + 1]->n;
+    M.small_bytes += 2.0 * stream_bytes(V.A) + stream_bytes(V.R) + stream_bytes(V.P) +
+                     (11.0 * n + 2.0 * nn) * w;
+  }
   M.small_nops = count;
   M.small_ctas = o.ctas;
   M.small_from = t;

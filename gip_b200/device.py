@@ -179,10 +179,10 @@ def pcg_params(mode: str = "fixed", maxit: int = 100, tol: float = 1e-6,
 
 # how a solve runs (GIPB200_SOLVE_*)
 SOLVE_FORMS = ("loop", "block", "cluster", "grid", "stream", "precond_cluster", "precond_grid")
-CYCLE_KINDS = ("jacobi0", "residual", "restrict", "dense", "prolong", "smooth", "tail")
+CYCLE_KINDS = ("jacobi0", "residual", "restrict", "dense", "prolong", "smooth", "tail", "small")
 # the kernel each product form runs as (GIPB200_FORM_*)
 FORM_KERNELS = ("k_amgp_spmv", "k_amg_spmv", "k_amg_spmv_pf", "k_amg_csr", "k_amg_dense",
-                "k_amg_jacobi0", "k_amg_tail", "k_amg_smooth_dot")
+                "k_amg_jacobi0", "k_amg_tail", "k_amg_smooth_dot", "k_amg_small")
 
 
 def _vcycle_profile(fn: str, handle, reps: int, stream) -> list:

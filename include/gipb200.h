@@ -241,7 +241,9 @@ int gipb200_pcg_kernel_time(gipb200_pcg S, int reps, void* stream, double* avg_m
  * kernel of one cycle in launch order: its level, its kind (GIPB200_CYCLE_*), its mean
  * time in ms and its algorithmic bytes (stored operator words once, every vector read
  * or written once).  At most `cap` kernels are written; *n_kernels = kernels per cycle.
- * Leaves the solution untouched; solve once first so the residual is set. */
+ * Leaves the solution untouched; solve once first so the residual is set.  The cycle is the
+ * one of a solve that runs kernel by kernel; a solve in one launch runs the same products
+ * without kernels of their own. */
 enum {
   GIPB200_CYCLE_JACOBI0 = 0,   /* x = D^-1 b (pre-smoothing from zero)           */
   GIPB200_CYCLE_RESIDUAL = 1,  /* t = b - A x                                    */
@@ -249,7 +251,9 @@ enum {
   GIPB200_CYCLE_DENSE = 3,     /* coarsest level: x = A^-1 b (dense inverse)     */
   GIPB200_CYCLE_PROLONG = 4,   /* x += P x_coarse                                */
   GIPB200_CYCLE_SMOOTH = 5,    /* x + D^-1 (b - A x) (level 0: with r.z)         */
-  GIPB200_CYCLE_TAIL = 6       /* the small levels and the coarsest, one launch  */
+  GIPB200_CYCLE_TAIL = 6,      /* the small levels and the coarsest, one launch  */
+                               /* over a grid (opt-in)                           */
+  GIPB200_CYCLE_SMALL = 7      /* the same levels in one launch of one cluster   */
 };
 int gipb200_pcg_vcycle_profile(gipb200_pcg S, int reps, void* stream, int cap, int* n_kernels,
                                int* h_level, int* h_kind, double* h_ms, double* h_bytes);
@@ -264,7 +268,8 @@ enum {
   GIPB200_FORM_DENSE = 4,      /* dense inverse of the coarsest level (k_amg_dense)       */
   GIPB200_FORM_VECTOR = 5,     /* element-wise (k_amg_jacobi0)                            */
   GIPB200_FORM_TAIL = 6,       /* the coarse tail in one launch (k_amg_tail)              */
-  GIPB200_FORM_SMOOTH_DOT = 7  /* level-0 smoothing with r.z, plain layout                */
+  GIPB200_FORM_SMOOTH_DOT = 7, /* level-0 smoothing with r.z, plain layout                */
+  GIPB200_FORM_SMALL = 8       /* the small levels in one cluster launch (k_amg_small)    */
 };
 int gipb200_pcg_vcycle_forms(gipb200_pcg S, int cap, int* n_kernels, int* h_form);
 
