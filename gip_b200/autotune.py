@@ -7,7 +7,9 @@ with its own grid.  For each operator size class the tuner times the engine's ow
 kernels (CUDA events over live launches, ``gipb200_dns_kernel_time``) for a few grid sizes
 (multiples of the SM count): first the SpMV grid, then, in the mixed form, the update's
 grid, and keeps the fastest of each.  The slice height (32 rows, one warp) and the block
-(256 threads) are fixed by the sliced layout and the reductions.  Results are cached per
+(256 threads) are fixed by the sliced layout and the reductions.  The grids are those of the
+kernel-by-kernel loop: an engine whose solves run as one launch has nothing to gain here.
+Results are cached per
 (kernel, rows, nnz) in memory and, if ``path`` is given, in a JSON file.
 
 For a batch solved by the persistent launch (``tune_batch``) the tuner times whole batch

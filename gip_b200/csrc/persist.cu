@@ -23,8 +23,9 @@
 // (host-driven), 128^3 32.5 against 84.
 // Element operations are GIP's (no FMA contraction); only the order of the dot products' sums
 // differs from the other forms.  Columns of ghost cells hold stored zeros in these operators
-// (checked at set-up): they enter the initial residual like every column, and the iterations,
-// where their entries of p stay fixed, drop them.
+// (checked at set-up; a later change of the values ends these forms, Pcg::follow_values): they
+// enter the initial residual like every column, and the iterations, where their entries of p
+// stay fixed, drop them.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

@@ -425,8 +425,9 @@ int gipb200_dns_snapshot(gipb200_dns E, int restore, void* stream);
 
 /* Launch shape of the PCG kernels (SpMV+dot grid, vector-kernel grid; 0 = default,
  * at most 8192 blocks of 256 threads).  A different shape changes the order of the
- * dot-product partial sums (results stay deterministic for a given shape).  The next
- * step re-captures its graph. */
+ * dot-product partial sums (results stay deterministic for a given shape).  Solves that run
+ * as one launch have a shape of their own, which this leaves alone (the mixed form's residual
+ * sum keeps the order of spmv_blocks).  The next step re-captures its graph. */
 int gipb200_dns_set_launch(gipb200_dns E, int spmv_blocks, int vec_blocks);
 
 /* gipb200_pcg_share_gpu for the engine's pressure solver: on != 0 for engines that advance side
@@ -461,7 +462,8 @@ enum {
 /* Times `reps` back-to-back launches of one PCG kernel on the engine's resident operator
  * with CUDA events on `stream`; returns the mean launch time and the kernel's compulsory
  * bytes per launch (stored values and indices read once, the vector read once, the
- * product written once).  Leaves the engine's fields untouched. */
+ * product written once).  These are the kernels of the kernel-by-kernel loop, whatever form
+ * the engine's solves take.  Leaves the engine's fields untouched. */
 int gipb200_dns_kernel_time(gipb200_dns E, int kernel, int reps, void* stream, double* avg_ms,
                             double* bytes);
 
@@ -481,7 +483,10 @@ int gipb200_batch_instance(gipb200_batch B, int i, gipb200_dns* out);
 /* nsteps timesteps of every instance, one graph launch each, on `stream`. */
 int gipb200_batch_advance(gipb200_batch B, int nsteps, void* stream);
 /* How the batch solves its pressure systems.  persistent = 0 (the default): inside each
- * instance's graph branch, as a single instance does.  persistent = 1: one cooperative
+ * instance's graph branch, or, when every instance is MIXED with AMG and the systems are small,
+ * all of them in one cooperative launch of a CTA group each.  Instances equal the same case
+ * run alone to the rounding of the dot products (in the branches no solve claims every SM, so
+ * GRID, STREAM and PRECOND_GRID solves run kernel by kernel).  persistent = 1: one cooperative
  * launch per timestep solves every instance's system, the launch's CTAs split into one
  * group per instance (shares set by gipb200_batch_balance); each group runs its instance's
  * mixed-form Jacobi-PCG and leaves when that instance has converged.  Needs every instance
