@@ -1548,6 +1548,7 @@ int gipb200_dns_share_gpu(gipb200_dns Dh, int on) {
   if (!Dh) return fail(GIPB200_ERR_ARG, "null engine");
   Dns& E = Dh->E;
   if (E.pcg.shared_gpu != (on != 0)) {
+    GIPB_CUDA(cudaDeviceSynchronize());  // a launched graph may still run
     E.pcg.shared_gpu = on != 0;
     E.drop_graph();  // the next step captures the other form of the solve
   }
