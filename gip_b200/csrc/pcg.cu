@@ -1832,7 +1832,8 @@ int Pcg::result(cudaStream_t s, gipb200_pcg_result* out) {
   if (out) {
     out->iterations = prm.mode == GIPB200_PCG_MIXED ? h_sc->total_inner : h_sc->iter;
     out->outer = h_sc->outer;
-    out->status = h_sc->status;
+    // the scalars are those of the first CTA, whose own waits may all have ended
+    out->status = wait_gave_up() ? GIPB200_ERR_TIMEOUT : h_sc->status;
     out->rr = h_sc->rr;
     out->bb = h_sc->bb;
   }
@@ -1927,6 +1928,7 @@ int gipb200_pcg_solve(gipb200_pcg S, const double* b, double* x, const double* x
                       gipb200_pcg_result* res) {
   if (!S || !b || !x || !x0) return fail(GIPB200_ERR_ARG, "null argument");
   cudaStream_t s = as_stream(stream);
+  S->P.clear_gave_up();
   GIPB_TRY(S->P.enqueue(b, x, x0, s, true));
   GIPB_TRY(S->P.result(s, res));
   return GIPB200_OK;

@@ -354,7 +354,9 @@ int gipb200_dns_history(gipb200_dns E, int* steps_taken, double* h_time, double*
  * min(steps taken, max_steps) steps; *steps_out (may be NULL) = steps written.  Synchronises
  * the device.  After a TIMEOUT (a device wait of a solve that runs as one launch gave up, after
  * about 2 s) the engine's state is not valid and further steps are refused with
- * GIPB200_ERR_TIMEOUT until a snapshot is restored. */
+ * GIPB200_ERR_TIMEOUT until a snapshot is restored (in a batch, until
+ * gipb200_batch_solver_status has reported it), also where the wait was another thread block's
+ * than the one that stores the status. */
 int gipb200_dns_solve_status(gipb200_dns E, int max_steps, int* h_status, int* steps_out);
 /* Runs one-launch solves and a barrier that wait for a thread block that does not exist, on the
  * engine's solver: *h_status = GIPB200_ERR_TIMEOUT when each gave up (after about 20 ms here)
@@ -431,8 +433,8 @@ int gipb200_dns_snapshot(gipb200_dns E, int restore, void* stream);
 int gipb200_dns_set_launch(gipb200_dns E, int spmv_blocks, int vec_blocks);
 
 /* gipb200_pcg_share_gpu for the engine's pressure solver: on != 0 for engines that advance side
- * by side on several streams, whose steps then overlap.  The next step re-captures its graph.
- * (The instances of a batch need no such call.) */
+ * by side on several streams, whose steps then overlap.  Waits for the device; the next step
+ * re-captures its graph.  (Within a batch the instances need no such call.) */
 int gipb200_dns_share_gpu(gipb200_dns E, int on);
 
 /* Algorithmic bytes of each phase of one timestep, in the order of
